@@ -420,7 +420,7 @@ def run_candidates(args, rank: int, world: int) -> dict | None:
     plain = [context(c, "fp64", sid) for c in cands]
     # fast contexts: one stream each (the batch runs on the first one's)
     fast_streams = [torch.cuda.Stream() for _ in cands]
-    # (block ILU sweeps: one SM per solve, so the candidates' solves overlap)
+    # (block ILU sweeps: a few SMs per solve, so the candidates' solves overlap)
     fast = [context(c, args.fast_precision, st.cuda_stream, adjoint_precision="fp32", sweeps="block")
             for c, st in zip(cands, fast_streams)]
     batch = Batch(fast)
@@ -559,7 +559,7 @@ def run_candidates(args, rank: int, world: int) -> dict | None:
             "viscosity": 1.8e-5,
             "fast": f"batched time loop ({args.fast_precision} residual, FP64 state); then all candidates' "
                     f"adjoints concurrently (own stream each), warm start {'on' if ws else 'off'}, block-ILU(0) "
-                    "BiCGSTAB (block sweeps, one SM each) with FP32 J^T products and FP64 true-residual restarts; "
+                    "BiCGSTAB (block sweeps, up to 8 SMs each) with FP32 J^T products and FP64 true-residual restarts; "
                     "FP64 forces/J/gradient",
             "plain": "FP64 residual (bit-exact), one context at a time, block-ILU(0) BiCGSTAB from zero "
                      "(sweeps chosen by size for a solve alone)",

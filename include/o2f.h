@@ -95,11 +95,11 @@ typedef enum o2f_status {
  * and objective differentiated, the limiter's own derivative left out). */
 #define O2F_JAC_FROZEN 2
 
-/* Triangular sweeps of the block ILU(0) preconditioner.  BLOCK: one thread
- * block walks the dependency levels (one SM per sweep: best when several
- * contexts solve at once, and alone on small meshes); WAITING: persistent
- * warps on up to 64 SMs, each row waiting on its dependencies (best alone on
- * large meshes); AUTO: BLOCK up to 200,000 cells, else WAITING. */
+/* Triangular sweeps of the block ILU(0) preconditioner.  BLOCK: a cluster of
+ * 1 to 8 thread blocks (by size) walks a schedule of the rows; WAITING:
+ * persistent warps on up to 64 SMs, each row waiting on its dependencies;
+ * AUTO: BLOCK.  A mesh whose schedule does not fit the blocks' shared memory
+ * is swept by WAITING. */
 #define O2F_SWEEPS_AUTO 0
 #define O2F_SWEEPS_BLOCK 1
 #define O2F_SWEEPS_WAITING 2

@@ -116,11 +116,17 @@ struct IluDev {
   int32_t* pos;       // [nc] position of the cell in the ILU order
   int32_t* order;     // [nc] cell at each ILU position (inverse of pos)
   int32_t* sweep;     // [2*nc] processing orders of the forward, then the backward sweep
-  int32_t* lev_off;   // [n_lo+1 + n_up+1] level offsets into the forward, then the backward order
-  int32_t* rec;       // [2*nc*8] block-sweep records per sweep position (row, dependency positions, slots)
-  Vec4<double>* out_f;  // [nc] block sweeps: forward values by forward position
-  Vec4<double>* out_b;  // [nc] block sweeps: backward values by backward position
-  double* pack;       // block sweeps: factor blocks in sweep order, interleaved over 32 positions (k_ilu_pack)
+  // cluster sweeps (sweep_plan.hpp, k_ilu_sweep_cluster), [0] forward, [1] backward
+  int cl_blocks;        // thread blocks per cluster
+  int cl_nlev[2];       // levels
+  int cl_chunks[2];     // 32-position chunks
+  int32_t* cl_info[2];  // [nlev*blocks*4] chunks and expected bytes of each level and block
+  int32_t* cl_rec[2];   // [32*chunks*kSweepRec] records by position
+  int32_t* cl_pos;      // [nc] forward position of each row
+  double* pack[2];      // [chunks*2048] factor blocks in sweep order (k_ilu_pack)
+  double* packD;        // [chunks*512] D^-1 in backward order
+  Vec4<double>* own_f;  // [32*chunks] input by forward position
+  Vec4<double>* own_b;  // [32*chunks] forward values by backward position
   double* A;          // [nc*5*16] row blocks (diagonal, then the 4 slots), row-major 4x4
   double* Dinv;       // [nc*16]
   int32_t* lo_cells;  // [nc] factorization levels, concatenated (offsets kept on the host)

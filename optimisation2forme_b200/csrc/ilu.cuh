@@ -23,6 +23,7 @@
 #pragma once
 
 #include "kernels.cuh"
+#include "sweep_plan.hpp"
 
 namespace o2f {
 
@@ -376,116 +377,101 @@ __global__ void __launch_bounds__(kSweepBlock) k_ilu_sweep(int n, IluDev ilu, co
   }
 }
 
-// One thread block solves a whole triangle, level after level: the rows of a
-// level are independent and a __syncthreads separates the levels, so no row
-// ever waits on a flag.  Each sweep position has a record (row, the sweep
-// positions of its dependencies, their slots); values are kept by sweep
-// position, and the last kSweepWindow of them also in shared memory, where
-// a row finds its dependencies -- they lie mostly a few levels back.  A
-// dependency q is read from shared memory when q >= e - kSweepWindow (e:
-// end of the current level): its slot is not overwritten by this level's
-// writes, which reuse the slots of positions [b - W, e - W).
-// The arithmetic of a row (dependencies in slot order) is that of
-// k_ilu_sweep: both give the same bits.  One SM per sweep, so the sweeps of
-// many contexts run side by side.
-constexpr int kSweepCtaThreads = 512;
-constexpr int kSweepWindow = 2048;  // values kept in shared memory (64 KiB; ~96 % of the dependencies)
-// Factor blocks of the next level staged in shared memory (two buffers,
-// alternating by level): dependency slots 0 and 1 of each position (on
-// triangles a forward row has at most 2 dependencies, a backward row rarely
-// 3) for the first 10 chunks of 32 positions forward (8 KiB each), the first
-// 6 backward with their D^-1 (4 KiB each) after them.
-constexpr int kStageSlots = 2;
+// One cluster of thread blocks solves a whole triangle, level after level
+// (sweep_plan.hpp: the levels, the rows of each block, and where each solved
+// value goes).  What bounds a sweep is the latency of a level -- about 500 of
+// them for 75k rows, each a dot of a few dozen terms -- so a level's path has
+// nothing on it but operand read, dot, and the way of the value to the rows
+// that need it:
+//   * a solved value is stored straight into the operand slots of the rows
+//     that need it, in the shared memory of their blocks, by st.async, whose
+//     bytes count on the barrier of the level that waits for them: no fence,
+//     no barrier over the cluster per level (only one every kSweepSkew / 2
+//     levels, arrived at that long before it is waited for, which bounds how
+//     far blocks run apart and so makes slots and barriers reusable);
+//   * factor blocks, D^-1 (backward), own values and records of the next
+//     kStageRing levels are copied into shared memory by a warp of its own
+//     (bulk copies, contiguous in sweep order), and are in a row's registers
+//     before the level begins.
+// Four lanes solve a row (one component each), eight warps the kSweepChunks
+// chunks of a block.  The arithmetic of a row (dependencies in slot order)
+// is that of k_ilu_sweep: both give the same bits.
+// Measured on B200, ms per adjoint iteration (four sweeps) alone: 1.08 at
+// 74,528 rows, 2.29 at 300,300, against 3.93 and 13.1 for one block walking
+// plain levels behind a block barrier and 5.2 and 11.6 for k_ilu_sweep; about
+// 1,000 cycles a level, of them 270 (forward) to 390 (backward) the dot and
+// some 600 from store to reader.  Slower, and not kept: a cluster barrier
+// with release per level (3.0 ms at 74,528 rows: the release waits for the
+// level's global stores, 1,400 cycles), operand slots that are polled for a
+// sentinel instead of barriers that are waited on (1.27 ms), 16-byte instead
+// of 8-byte stores per lane (1.18 against 1.13 ms).
+constexpr int kSweepThreads = 128 * kSweepChunks + 32 * (kSweepChunks + 2);
+constexpr int kSweepWindow = 2048;  // operand slots (32 B each)
+static_assert(kSweepWindow == kSweepSlots && (kSweepSlots & (kSweepSlots - 1)) == 0, "operand slots");
+constexpr int kStageSlots = 3;      // dependencies whose blocks are staged (the third where a row of the chunk has one)
 constexpr int kStageChunkDoubles = kStageSlots * 512;
-constexpr int kStageChunksFwd = 10;
-constexpr int kStageChunksBwd = 6;
+constexpr int kStageChunksFwd = 2;
+constexpr int kStageChunksBwd = 2;
+static_assert(kStageChunksFwd == kSweepChunks && kStageChunksBwd == kSweepChunks, "every chunk of a block is staged");
 constexpr int kStageBwdD = kStageChunksBwd * kStageChunkDoubles;  // offset of the staged D^-1, doubles
-constexpr int kStageDoubles = kStageChunksFwd * kStageChunkDoubles;  // one buffer (backward: 6*1024 + 6*512)
-constexpr size_t kSweepSmem = sizeof(Vec4<double>) * kSweepWindow + 2 * kStageDoubles * sizeof(double);
+constexpr int kStageDoubles = kStageBwdD + kStageChunksBwd * 512;  // blocks (and D^-1) of one level
+constexpr int kStageRing = 4;       // levels staged at once
+constexpr int kStageOwn = kSweepChunks * 128;  // own values of one level, doubles
+constexpr int kRecChunkBytes = 32 * kSweepRec * 4;
+constexpr int kL2Lead = 16;         // levels between the L2 prefetch of a level's blocks and its use
+constexpr int kSweepBlockBytes = kStageRing * kStageDoubles * 8;
+constexpr int kSweepOwnBytes = kStageRing * kStageOwn * 8;
+constexpr int kSweepRecBytes = kStageRing * kSweepChunks * kRecChunkBytes;
+// operand slots, blocks, own values + records + mbarriers + chunk counts
+constexpr size_t kSweepSmem = sizeof(Vec4<double>) * kSweepWindow + 4 * kStageDoubles * sizeof(double) + 20688;
+static_assert(kSweepSmem == 32 * kSweepWindow + kSweepBlockBytes + kSweepOwnBytes + kSweepRecBytes +
+                                8 * (kSweepBars + 2 * kStageRing) + 4 * kStageRing,
+              "shared memory of a sweep block");
 static_assert(kSweepSmem <= 227 * 1024, "block sweep shared memory above the per-block limit");
 static_assert(kStageBwdD + kStageChunksBwd * 512 <= kStageDoubles, "backward staging overflows its buffer");
+constexpr int kSweepWaitLimit = 1 << 20;  // polls of an mbarrier (up to 1 us each) before the sweep gives up
 
-// Factor blocks of the block sweeps, repacked in sweep order after every
-// factorization and interleaved over 32 consecutive positions, so that the
-// 32 lanes of a warp (consecutive positions of a level) read 32 consecutive
-// doubles per element: element e of dependency d of position p of direction
-// dir is pk[dir*n*64 + (p>>5)*2048 + d*512 + e*32 + (p&31)] (n rounded up to
-// 32), D^-1 of backward position p is pk[2*n*64 + (p>>5)*512 + e*32 + (p&31)].
-__device__ __forceinline__ int64_t sweep_pack_base(int64_t n32, int dir, int p) {
-  return (int64_t)dir * n32 * 64 + (int64_t)(p >> 5) * 2048 + (p & 31);
+// Place of element el of the block at lane q inside its 512 doubles: the two
+// halves of a block row, then (row, component), so that a warp's four lanes
+// per row read 16 consecutive bytes each, all 32 lanes 512.
+__host__ __device__ __forceinline__ int sweep_pack_place(int q, int el) {
+  return ((el >> 1) & 1) * 256 + (q * 4 + (el >> 2)) * 2 + (el & 1);
 }
 
-__global__ void k_ilu_pack(int n, IluDev ilu) {
-  const int64_t n32 = ((int64_t)n + 31) / 32 * 32;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // (dir, p, d) with d = 4 for D^-1
-  if (t >= (int64_t)2 * n * 5) return;
-  const int dir = (int)(t / ((int64_t)n * 5));
-  const int64_t rest = t % ((int64_t)n * 5);
-  const int p = (int)(rest / 5), d = (int)(rest % 5);
-  const int* rec = ilu.rec + 8 * ((int64_t)dir * n + p);
+// Factor blocks in sweep order, repacked after every factorization: dependency
+// d of position p of direction dir at pack[dir] + (p >> 5) * 2048 + d * 512 +
+// sweep_pack_place(p & 31, .), D^-1 of backward position p at packD +
+// (p >> 5) * 512 + the same.  One thread per two consecutive doubles written.
+__global__ void __launch_bounds__(256) k_ilu_pack(IluDev ilu) {
+  const int64_t nf = (int64_t)ilu.cl_chunks[0] * 1024, nb = (int64_t)ilu.cl_chunks[1] * 1024,
+                nd = (int64_t)ilu.cl_chunks[1] * 256;
+  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nf + nb + nd) return;
+  const int kind = t < nf ? 0 : t < nf + nb ? 1 : 2;
+  t -= kind == 0 ? 0 : kind == 1 ? nf : nf + nb;
+  const int per = kind == 2 ? 256 : 1024;
+  const int64_t chunk = t / per;
+  const int d = (int)(t % per) >> 8, in = (int)(t & 255);
+  const int half = in >> 7, q = (in >> 2) & 31, c = in & 3;
+  const int32_t* rec = ilu.cl_rec[kind == 0 ? 0 : 1] + (chunk * 32 + q) * kSweepRec;
   const int row = rec[0];
-  if (d == 4) {
-    if (dir == 0) return;
-    const double* D = ilu.Dinv + (int64_t)row * 16;
-    double* dst = ilu.pack + 2 * n32 * 64 + (int64_t)(p >> 5) * 512 + (p & 31);
-#pragma unroll
-    for (int e = 0; e < 16; ++e) dst[e * 32] = D[e];
-    return;
+  if (row < 0) return;
+  const double* src;
+  double* dst;
+  if (kind == 2) {
+    src = ilu.Dinv + (int64_t)row * 16;
+    dst = ilu.packD + chunk * 512;
+  } else {
+    if (d >= rec[1]) return;
+    const int slot = (int)(((unsigned int)rec[9] >> (8 * d)) & 0xff);
+    src = ilu.A + (int64_t)row * 80 + 16 * (1 + slot);
+    dst = ilu.pack[kind] + chunk * 2048 + d * 512;
   }
-  if (rec[1 + d] < 0) return;
-  const int slot = (int)(((unsigned int)rec[5] >> (8 * d)) & 0xff);
-  const double* B = ilu.A + (int64_t)row * 80 + 16 * (1 + slot);
-  double* dst = ilu.pack + sweep_pack_base(n32, dir, p) + d * 512;
-#pragma unroll
-  for (int e = 0; e < 16; ++e) dst[e * 32] = B[e];
+  *reinterpret_cast<double2*>(dst + sweep_pack_place(q, 4 * c + 2 * half)) =
+      *reinterpret_cast<const double2*>(src + 4 * c + 2 * half);
 }
 
-// One row of a block sweep: own value minus the dependencies' products
-// (slot order), times D^-1 backward; stored in the window, by position, and
-// (backward) into z by row.  Factor blocks of the level's first `nch` chunks
-// (from chunk c0) are read from the staged copy `stage`, the rest from the
-// packed copy in global memory: same layout, same values.
-template <bool kForward>
-__device__ __forceinline__ void sweep_cta_row(const IluDev& ilu, int p, int e, const int4& a, const int4& c,
-                                              Vec4<double> acc, const Vec4<double>* win_r, Vec4<double>* win,
-                                              Vec4<double>* out, Vec4<double>* z, const double* stage, int c0,
-                                              int nch) {
-  const int i = a.x;
-  const int dq[4] = {a.y, a.z, a.w, c.x};
-  const int64_t n32 = ((int64_t)ilu.nc + 31) / 32 * 32;
-  const int k = (p >> 5) - c0;  // >= 0: p lies in the level that starts in chunk c0
-  const bool staged = k < nch;
-  const double* P = ilu.pack + sweep_pack_base(n32, kForward ? 0 : 1, p);
-  const double* S = stage + k * kStageChunkDoubles + (p & 31);
-#pragma unroll
-  for (int d = 0; d < 4; ++d) {
-    const int q = dq[d];
-    if (q < 0) break;
-    const double* Bk = (staged && d < kStageSlots ? S : P) + d * 512;  // element k at Bk[32 k]
-    const Vec4<double> v = q >= e - kSweepWindow ? win_r[q % kSweepWindow] : out[q];
-    acc.a -= Bk[0] * v.a + Bk[32] * v.b + Bk[64] * v.c + Bk[96] * v.d;
-    acc.b -= Bk[128] * v.a + Bk[160] * v.b + Bk[192] * v.c + Bk[224] * v.d;
-    acc.c -= Bk[256] * v.a + Bk[288] * v.b + Bk[320] * v.c + Bk[352] * v.d;
-    acc.d -= Bk[384] * v.a + Bk[416] * v.b + Bk[448] * v.c + Bk[480] * v.d;
-  }
-  if (!kForward) {
-    const double* D = staged ? stage + kStageBwdD + k * 512 + (p & 31)
-                             : ilu.pack + 2 * n32 * 64 + (int64_t)(p >> 5) * 512 + (p & 31);
-    Vec4<double> o4;
-    o4.a = D[0] * acc.a + D[32] * acc.b + D[64] * acc.c + D[96] * acc.d;
-    o4.b = D[128] * acc.a + D[160] * acc.b + D[192] * acc.c + D[224] * acc.d;
-    o4.c = D[256] * acc.a + D[288] * acc.b + D[320] * acc.c + D[352] * acc.d;
-    o4.d = D[384] * acc.a + D[416] * acc.b + D[448] * acc.c + D[480] * acc.d;
-    acc = o4;
-  }
-  const Vec4<double> v{__longlong_as_double((long long)sweep_bits(acc.a)),
-                       __longlong_as_double((long long)sweep_bits(acc.b)),
-                       __longlong_as_double((long long)sweep_bits(acc.c)),
-                       __longlong_as_double((long long)sweep_bits(acc.d))};
-  win[p % kSweepWindow] = v;
-  out[p] = v;
-  if (!kForward) z[i] = v;
-}
+__device__ __forceinline__ uint32_t sweep_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Bulk prefetch of [p, p + bytes) into L2 (a hint: no data is returned and
 // no completion is awaited); p 16-byte aligned, bytes a multiple of 16.
@@ -493,144 +479,248 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* p, uint32_t bytes) 
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// The L2 prefetch of one level [b, e) of a block sweep, by one warp: the
-// 32-position chunks of packed factor blocks that hold it (16 KiB each, plus
-// 4 KiB of D^-1 backward) and its records (32 B per position).  The chunks
-// lie inside the packed copy (n rounded up to 32 positions), the records
-// inside the 2n records of the two directions.
-template <bool kForward>
-__device__ __forceinline__ void sweep_prefetch_level(const IluDev& ilu, const int* rec, int b, int e, int lane) {
-  if (b >= e) return;
-  const int64_t n32 = ((int64_t)ilu.nc + 31) / 32 * 32;
-  for (int c = (b >> 5) + lane; c <= ((e - 1) >> 5); c += 32) {
-    prefetch_l2_bulk(ilu.pack + (kForward ? 0 : n32 * 64) + (int64_t)c * 2048, 2048 * sizeof(double));
-    if (!kForward) prefetch_l2_bulk(ilu.pack + 2 * n32 * 64 + (int64_t)c * 512, 512 * sizeof(double));
-  }
-  const char* r0 = reinterpret_cast<const char*>(rec + 8 * (int64_t)b);
-  const int64_t bytes = (int64_t)(e - b) * 8 * sizeof(int);
-  for (int64_t o = (int64_t)lane * 4096; o < bytes; o += 32 * 4096)
-    prefetch_l2_bulk(r0 + o, (uint32_t)(bytes - o < 4096 ? bytes - o : 4096));
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 
-// Asynchronous 16-byte global -> shared copy (completes at cp_async_wait_all).
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Chunks of 32 positions of the level [b, e) that are staged.
-template <bool kForward>
-__device__ __forceinline__ int sweep_stage_chunks(int b, int e) {
-  if (b >= e) return 0;
-  const int n = ((e - 1) >> 5) - (b >> 5) + 1;
-  const int cap = kForward ? kStageChunksFwd : kStageChunksBwd;
-  return n < cap ? n : cap;
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-
-// Stage the factor blocks of level [b, e) into `buf`, by the whole block:
-// dependency slots 0 .. kStageSlots-1 of the level's first chunks (the
-// leading kStageChunkDoubles of each 2048-double chunk), and D^-1 backward.
-// Each copied chunk lies inside the packed copy (chunk indices up to
-// (e - 1) >> 5 < n32 / 32); addresses and sizes are multiples of 16 bytes.
-template <bool kForward>
-__device__ __forceinline__ void sweep_stage_level(const IluDev& ilu, int b, int e, double* buf, int t, int T) {
-  const int nch = sweep_stage_chunks<kForward>(b, e);
-  if (nch == 0) return;
-  const int64_t n32 = ((int64_t)ilu.nc + 31) / 32 * 32;
-  const double* src = ilu.pack + (kForward ? 0 : n32 * 64) + (int64_t)(b >> 5) * 2048;
-  constexpr int kPieces = kStageChunkDoubles / 2;  // 16-byte pieces per staged chunk
-  for (int k = t; k < nch * kPieces; k += T) {
-    const int ch = k / kPieces, pc = k - ch * kPieces;
-    cp_async16(buf + ch * kStageChunkDoubles + 2 * pc, src + (int64_t)ch * 2048 + 2 * pc);
-  }
-  if (!kForward) {
-    const double* srcD = ilu.pack + 2 * n32 * 64 + (int64_t)(b >> 5) * 512;
-    for (int k = t; k < nch * 256; k += T) cp_async16(buf + kStageBwdD + 2 * k, srcD + 2 * k);
-  }
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Whether the phase has completed; sleeps up to a microsecond for it.
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(1000)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait for the phase of an mbarrier; once one has run out (bad), none
+// waits any more.
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& bad) {
+  if (bad) return;
+  for (int i = 0; i < kSweepWaitLimit; ++i)
+    if (bar_try(bar, parity)) return;
+  bad = true;
 }
 
-// The first two rows of each thread in a level are software-pipelined: their
-// records are loaded during the level before and their own values (r, or the
-// forward value) requested at its end, so a level starts with its operands
-// in flight; further rows load at use.  Factor blocks come from the packed
-// copy (k_ilu_pack), coalesced across the warp: the first chunks of each
-// level staged in shared memory by asynchronous copies issued during the
-// level before (two buffers), the rest read from global memory.  The first
-// warp also requests the blocks and records of the level two ahead into L2
-// as each level starts, for when other contexts' sweeps and products have
-// evicted them.  One block per SM is declared so that the compiler keeps the
-// rows' loads in registers (about 100 per thread) instead of capping them.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
+// r (in forward sweep order, ilu.own_f) -> ilu.own_b (kForward), ilu.own_b ->
+// z (backward).  Grid: one cluster.  Every wait on an mbarrier is bounded;
+// when one runs out the sweep records sync->err, waits on none any more, uses
+// nothing it waited for, and still takes part in every cluster barrier.
 template <bool kForward>
-__global__ void __launch_bounds__(kSweepCtaThreads, 1) k_ilu_sweep_cta(int n, IluDev ilu, const Vec4<double>* r,
-                                                                    Vec4<double>* z, const int* gate) {
+__global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev ilu, Vec4<double>* z, const int* gate) {
   if (gated(gate)) return;
-  extern __shared__ Vec4<double> win[];
-  const int* rec = ilu.rec + (kForward ? 0 : (int64_t)8 * n);
-  const int32_t* off = ilu.lev_off + (kForward ? 0 : ilu.n_lo + 1);
-  const int nlev = kForward ? ilu.n_lo : ilu.n_up;
-  Vec4<double>* out = kForward ? ilu.out_f : ilu.out_b;  // by sweep position
-  const int T = blockDim.x, t = threadIdx.x;
-  auto rec_a = [&](int p) { return *reinterpret_cast<const int4*>(rec + 8 * (int64_t)p); };
-  auto rec_c = [&](int p) { return *reinterpret_cast<const int4*>(rec + 8 * (int64_t)p + 4); };
-  auto own_of = [&](const int4& a, const int4& c) { return kForward ? r[a.x] : ilu.out_f[c.z]; };
-  double* stg = reinterpret_cast<double*>(win + kSweepWindow);  // 2 x kStageDoubles
-  int4 ra[2], rc[2];
-  Vec4<double> own[2];
-  if (t < 32)
-    for (int l = 0; l < 2 && l < nlev; ++l) sweep_prefetch_level<kForward>(ilu, rec, off[l], off[l + 1], t);
-  if (nlev > 0) {
-    sweep_stage_level<kForward>(ilu, off[0], off[1], stg, t, T);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int p = off[0] + t + k * T;
-      if (p < off[1]) {
-        ra[k] = rec_a(p);
-        rc[k] = rec_c(p);
-        own[k] = own_of(ra[k], rc[k]);
-      }
+  constexpr int kDir = kForward ? 0 : 1;
+  extern __shared__ __align__(128) unsigned char sweep_sm[];
+  double* s_blk = reinterpret_cast<double*>(sweep_sm);
+  double* s_own = reinterpret_cast<double*>(sweep_sm + kSweepBlockBytes);
+  unsigned char* s_op = sweep_sm + kSweepBlockBytes + kSweepOwnBytes;
+  unsigned char* s_rec = s_op + 32 * kSweepWindow;
+  const uint32_t bar_op = sweep_smem(s_rec + kSweepRecBytes);  // values of a level
+  const uint32_t bar_full = bar_op + 8 * kSweepBars;           // staged copies of a level
+  const uint32_t bar_empty = bar_full + 8 * kStageRing;        // its last reader
+  int* s_cnt = reinterpret_cast<int*>(s_rec + kSweepRecBytes + 8 * (kSweepBars + 2 * kStageRing));
+  const int nlev = ilu.cl_nlev[kDir];
+  const int C = (int)gridDim.x, rank = (int)blockIdx.x;
+  const int4* __restrict__ info = reinterpret_cast<const int4*>(ilu.cl_info[kDir]) + rank;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kSweepBars; ++i) bar_init(bar_op + 8u * i, 1);
+    for (int i = 0; i < kStageRing; ++i) {
+      bar_init(bar_full + 8u * i, kSweepChunks);
+      bar_init(bar_empty + 8u * i, 4 * kSweepChunks);
     }
-    cp_async_wait_all();
-    __syncthreads();
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int l = 0; l < nlev; ++l) {
-    const int b = off[l], e = off[l + 1];
-    const int ne = l + 1 < nlev ? off[l + 2] : e;
-    if (t < 32 && l + 2 < nlev) sweep_prefetch_level<kForward>(ilu, rec, ne, off[l + 3], t);
-    // this level's staged blocks (filled during the level before); the next
-    // level's into the other buffer, whose last readers passed the barrier
-    const double* cur = stg + (l & 1) * kStageDoubles;
-    const int c0 = b >> 5, nch = sweep_stage_chunks<kForward>(b, e);
-    if (l + 1 < nlev) sweep_stage_level<kForward>(ilu, e, ne, stg + ((l + 1) & 1) * kStageDoubles, t, T);
-    int4 na[2], nc[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {  // the next level's records, in flight during this one
-      const int q = e + t + k * T;
-      if (q < ne) {
-        na[k] = rec_a(q);
-        nc[k] = rec_c(q);
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // all blocks run, their mbarriers are set up
+  bool bad = false;
+  // Before level 4 i a warp arrives for the i-th time, once all have arrived
+  // for the (i-1)-th: at level l every level up to l - kSweepSkew has been
+  // left.  (Relaxed: what a warp read of those levels it has used by then.)
+  auto keep_together = [&](int l) {
+    if (l % (kSweepSkew / 2)) return;
+    __syncwarp();
+    if (l > 0) cluster_wait();
+    cluster_arrive();
+  };
+
+  // Helper warps, one thread of each at work: one per chunk that stages its
+  // copies, one that sets what each level's barrier waits for, one that
+  // requests blocks into L2 (a single thread for all took longer than a level).
+  if (warp >= 4 * kSweepChunks) {
+    const int32_t* __restrict__ rec = ilu.cl_rec[kDir];
+    const double* __restrict__ pack = ilu.pack[kDir];
+    const double* own = reinterpret_cast<const double*>(kForward ? ilu.own_f : ilu.own_b);
+    const int j = warp - 4 * kSweepChunks;
+    // A level's barrier is set kSweepNear levels ahead: by then every warp
+    // has left the level that used it last (kSweepSkew levels back), so a
+    // phase that has nothing to wait for cannot pass one that is waited on.
+    const int kLead = j < kSweepChunks ? kStageRing : j == kSweepChunks ? kSweepNear : kL2Lead;
+    auto info_of = [&](int l) { return l < nlev ? info[(int64_t)l * C] : make_int4(0, -1, 0, 0); };
+    auto work = [&](int l, const int4& in) {
+      if (in.y < 0) return;
+      if (j < kSweepChunks) {
+        const int slot = l % kStageRing;
+        const uint32_t bar = bar_full + 8u * slot;
+        if (j == 0) s_cnt[slot] = in.y;
+        if (j >= in.y) {
+          bar_arrive(bar);
+          return;
+        }
+        const uint32_t blk = (in.z >> j & 1 ? 3 : 2) * 4096;
+        const int64_t k = in.x + (int64_t)j * C;
+        const uint32_t dst = sweep_smem(s_blk + slot * kStageDoubles);
+        bar_expect(bar, 1024 + kRecChunkBytes + (kForward ? 0 : 4096) + blk);
+        bulk_copy(dst + (uint32_t)j * kStageChunkDoubles * 8, pack + k * 2048, blk, bar);
+        if (!kForward) bulk_copy(dst + (uint32_t)(kStageBwdD + j * 512) * 8, ilu.packD + k * 512, 4096, bar);
+        bulk_copy(sweep_smem(s_rec) + (uint32_t)(slot * kSweepChunks + j) * kRecChunkBytes,
+                  rec + k * 32 * kSweepRec, kRecChunkBytes, bar);
+        bulk_copy(sweep_smem(s_own + slot * kStageOwn + j * 128), own + k * 128, 1024, bar);
+      } else if (j == kSweepChunks) {
+        bar_expect(bar_op + 8u * (l % kSweepBars), (uint32_t)in.w);
+      } else {
+        for (int i = 0; i < in.y; ++i) {
+          const int64_t k = in.x + (int64_t)i * C;
+          prefetch_l2_bulk(pack + k * 2048, 8192);
+          if (!kForward) prefetch_l2_bulk(ilu.packD + k * 512, 4096);
+        }
+      }
+    };
+    int4 next{};
+    if (lane == 0) {
+      for (int l = 0; l < kLead; ++l) work(l, info_of(l));
+      next = info_of(kLead);
+    }
+    for (int l = 0; l < nlev; ++l) {
+      keep_together(l);
+      if (lane == 0) {
+        const int4 in = next;
+        next = info_of(l + 1 + kLead);
+        if (j < kSweepChunks)
+          bar_wait(bar_empty + 8u * (l % kStageRing), (l / kStageRing) & 1, bad);
+        else if (j > kSweepChunks)
+          bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
+        if (!bad) work(l + kLead, in);
       }
     }
+  } else {
+    const int j = warp >> 2, q = (warp & 3) * 8 + (lane >> 2), c = lane & 3;
+    const uint32_t op_base = sweep_smem(s_op);
+    // a row's operands that do not depend on the level before, in registers
+    double2 b[2][2], dv[2];
+    double ow = 0.0;
+    int4 r0, tgt;
+    int posb = 0, cnt = 0;
+    auto load_row = [&](int l) {
+      const int slot = l % kStageRing;
+      bar_wait(bar_full + 8u * slot, (l / kStageRing) & 1, bad);
+      const double* s = s_blk + slot * kStageDoubles + (q * 4 + c) * 2;
+      const unsigned char* r = s_rec + (slot * kSweepChunks + j) * kRecChunkBytes + q * (kSweepRec * 4);
+      cnt = s_cnt[slot];
+      r0 = *reinterpret_cast<const int4*>(r);
+      tgt = *reinterpret_cast<const int4*>(r + 16);
+      if (kForward) posb = *reinterpret_cast<const int*>(r + 32);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int p = b + t + k * T;
-      if (p < e) sweep_cta_row<kForward>(ilu, p, e, ra[k], rc[k], own[k], win, win, out, z, cur, c0, nch);
-    }
-    for (int p = b + t + 2 * T; p < e; p += T) {
-      const int4 a = rec_a(p), c = rec_c(p);
-      sweep_cta_row<kForward>(ilu, p, e, a, c, own_of(a, c), win, win, out, z, cur, c0, nch);
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {  // the next level's operands, requested before the barrier
-      const int q = e + t + k * T;
-      if (q < ne) {
-        ra[k] = na[k];
-        rc[k] = nc[k];
-        own[k] = own_of(ra[k], rc[k]);
+      for (int d = 0; d < 2; ++d) {
+        b[d][0] = *reinterpret_cast<const double2*>(s + j * kStageChunkDoubles + d * 512);
+        b[d][1] = *reinterpret_cast<const double2*>(s + j * kStageChunkDoubles + d * 512 + 256);
       }
+      ow = s_own[slot * kStageOwn + j * 128 + q * 4 + c];
+      if (!kForward) {
+        dv[0] = *reinterpret_cast<const double2*>(s + kStageBwdD + j * 512);
+        dv[1] = *reinterpret_cast<const double2*>(s + kStageBwdD + j * 512 + 256);
+      }
+    };
+    load_row(0);
+    for (int l = 0; l < nlev; ++l) {
+      keep_together(l);
+      double acc = ow;
+      bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
+      const bool mine = !bad && j < cnt && r0.x >= 0;  // after a wait that ran out nothing is taken for a record
+      const int nd = mine ? r0.y : 0;
+      // both usual operands at once, whether the row has them or not
+      auto operand = [&](uint32_t slot, double2& x, double2& y) {
+        const double2* v = reinterpret_cast<const double2*>(s_op + (slot & (kSweepSlots - 1)) * 32);
+        x = v[0];
+        y = v[1];
+      };
+      double2 x, y, x1, y1;
+      operand((uint32_t)r0.z, x, y);
+      operand((uint32_t)r0.z >> 16, x1, y1);
+      const double s0 = b[0][0].x * x.x + b[0][0].y * x.y + b[0][1].x * y.x + b[0][1].y * y.y;
+      const double s1 = b[1][0].x * x1.x + b[1][0].y * x1.y + b[1][1].x * y1.x + b[1][1].y * y1.y;
+      if (nd > 0) acc -= s0;
+      if (nd > 1) acc -= s1;
+      if (nd > 2) {  // rare on triangles
+        const double* s = s_blk + (l % kStageRing) * kStageDoubles + j * kStageChunkDoubles + 1024 + (q * 4 + c) * 2;
+        const double2 bx = *reinterpret_cast<const double2*>(s), by = *reinterpret_cast<const double2*>(s + 256);
+        operand((uint32_t)r0.w, x, y);
+        acc -= bx.x * x.x + bx.y * x.y + by.x * y.x + by.y * y.y;
+        if (nd > 3) {  // quadrilaterals, at the end of an elimination front
+          const int64_t k = info[(int64_t)l * C].x + (int64_t)j * C;
+          const double* g = ilu.pack[kDir] + k * 2048 + 1536 + (q * 4 + c) * 2;
+          const double2 gx = *reinterpret_cast<const double2*>(g), gy = *reinterpret_cast<const double2*>(g + 256);
+          operand((uint32_t)r0.w >> 16, x, y);
+          acc -= gx.x * x.x + gx.y * x.y + gy.x * y.x + gy.y * y.y;
+        }
+      }
+      if (!kForward) {
+        const int g = lane & ~3;
+        __syncwarp();
+        const double a0 = __shfl_sync(0xffffffffu, acc, g), a1 = __shfl_sync(0xffffffffu, acc, g + 1),
+                     a2 = __shfl_sync(0xffffffffu, acc, g + 2), a3 = __shfl_sync(0xffffffffu, acc, g + 3);
+        acc = dv[0].x * a0 + dv[0].y * a1 + dv[1].x * a2 + dv[1].y * a3;
+      }
+      if (mine) {
+        const int tg[4] = {tgt.x, tgt.y, tgt.z, tgt.w};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          if (tg[t] < 0) break;  // the record's targets come first
+          uint32_t base;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base) : "r"(op_base), "r"(tg[t] >> 16));
+          const uint32_t va = base + (uint32_t)(tg[t] & 0xfff) * 32 + (uint32_t)c * 8;
+          const uint32_t ba = base + (bar_op - op_base) + (uint32_t)(tg[t] >> 12 & 15) * 8;
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(va),
+                       "l"(__double_as_longlong(acc)), "r"(ba)
+                       : "memory");
+        }
+      }
+      double* to = !mine ? nullptr
+                   : kForward ? reinterpret_cast<double*>(ilu.own_b) + (int64_t)posb * 4 + c
+                              : reinterpret_cast<double*>(z) + (int64_t)r0.x * 4 + c;
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar_empty + 8u * (l % kStageRing));
+      if (l + 1 < nlev) load_row(l + 1);
+      if (to) *to = acc;
     }
-    cp_async_wait_all();  // this thread's copies of the next level, visible to all after the barrier
-    __syncthreads();
+  }
+  __syncwarp();
+  cluster_wait();
+  cluster_arrive();
+  cluster_wait();  // no block leaves while another may still write into it
+  if (bad) {
+    atomicExch(&ilu.sync[kDir].err, 1);
+    // copies of the last levels may still be in flight
+    for (int l = nlev > kStageRing ? nlev - kStageRing : 0; l < nlev; ++l) {
+      bool late = false;
+      bar_wait(bar_full + 8u * (l % kStageRing), (l / kStageRing) & 1, late);
+    }
   }
 }
 

@@ -385,9 +385,11 @@ __global__ void __launch_bounds__(kBlock) k_bicg_start(int64_t n4, const double*
   }
 }
 
-// p = r + beta (p - omega v) (and r0 = r on a restart).
+// p = r + beta (p - omega v) (and r0 = r on a restart).  With pos, p also goes
+// to po in the order pos (the input of a block sweep).
 __global__ void __launch_bounds__(kBlock) k_bicg_p(int64_t n4, const double* __restrict__ r, double* __restrict__ r0,
                                                    double* __restrict__ p, const double* __restrict__ v,
+                                                   const int32_t* __restrict__ pos, double* __restrict__ po,
                                                    KrylovState* ks) {
   if (ks->stop) return;
   const double beta = ks->beta, omega = ks->omega;
@@ -395,7 +397,9 @@ __global__ void __launch_bounds__(kBlock) k_bicg_p(int64_t n4, const double* __r
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
     const double ri = r[i];
     if (restart) r0[i] = ri;
-    p[i] = ri + beta * (p[i] - omega * v[i]);
+    const double pi = ri + beta * (p[i] - omega * v[i]);
+    p[i] = pi;
+    if (pos) po[4 * (int64_t)pos[i >> 2] + (i & 3)] = pi;
   }
 }
 
@@ -424,14 +428,18 @@ __global__ void __launch_bounds__(kBlock) k_bicg_jt_v(int64_t nc, const int32_t*
   }
 }
 
-// s = r - alpha v.
+// s = r - alpha v (and to so in the order pos, as k_bicg_p).
 __global__ void __launch_bounds__(kBlock) k_bicg_s(int64_t n4, const double* __restrict__ r,
                                                    const double* __restrict__ v, double* __restrict__ s,
+                                                   const int32_t* __restrict__ pos, double* __restrict__ so,
                                                    KrylovState* ks) {
   if (ks->stop) return;
   const double alpha = ks->alpha;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x)
-    s[i] = r[i] - alpha * v[i];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
+    const double si = r[i] - alpha * v[i];
+    s[i] = si;
+    if (pos) so[4 * (int64_t)pos[i >> 2] + (i & 3)] = si;
+  }
 }
 
 // t = J^T shat (shat = M^{-1} s, or s itself without preconditioner) with the

@@ -661,41 +661,7 @@ void Solver::setup_ilu_host(const std::vector<int32_t>& jslot, const std::vector
     for (int64_t i = nc - 1; i >= 0; --i) ilu_sweep_h_[nc + fill[levu[order[i]]]++] = order[i];
   }
   ilu_n_up_ = nup;
-  // level offsets of both sweep orders, forward then backward
-  ilu_lev_off_h_.assign(lo_off_h_.begin(), lo_off_h_.end());
-  ilu_lev_off_h_.insert(ilu_lev_off_h_.end(), up_off.begin(), up_off.end());
-  // Records of the block sweeps, per sweep position p (8 int32): the row,
-  // the sweep positions of its dependencies in slot order (-1: none), their
-  // slots (8 bits each), and for the backward sweep the row's forward
-  // position (where its forward value is).
-  {
-    std::vector<int32_t> posf(nc), posb(nc);
-    for (int64_t p = 0; p < nc; ++p) {
-      posf[ilu_sweep_h_[p]] = (int32_t)p;
-      posb[ilu_sweep_h_[nc + p]] = (int32_t)p;
-    }
-    ilu_rec_h_.assign(16 * nc, -1);
-    for (int dir = 0; dir < 2; ++dir)
-      for (int64_t p = 0; p < nc; ++p) {
-        const int32_t c = ilu_sweep_h_[dir * nc + p];
-        int32_t* rec = ilu_rec_h_.data() + 8 * (dir * nc + p);
-        rec[0] = c;
-        int nd = 0;
-        uint32_t slots = 0xffffffffu;
-        for (int k = 0; k < 4; ++k) {
-          const int32_t o = nbr(c, k);
-          if (o < 0) continue;
-          const bool dep = dir == 0 ? ilu_pos_h_[o] < ilu_pos_h_[c] : ilu_pos_h_[o] > ilu_pos_h_[c];
-          if (!dep) continue;
-          rec[1 + nd] = dir == 0 ? posf[o] : posb[o];
-          slots = (slots & ~(0xffu << (8 * nd))) | ((uint32_t)k << (8 * nd));
-          ++nd;
-        }
-        rec[5] = (int32_t)slots;
-        rec[6] = posf[c];
-        rec[7] = 0;
-      }
-  }
+  ilu_plan_h_ = make_sweep_plan(nc, ilu_nbr_h_, ilu_pos_h_, order);
   ilu_order_h_ = std::move(order);
   ilu_.nc = nc;
   ilu_.n_lo = nlo;
@@ -715,11 +681,26 @@ void Solver::ilu_factor() {
     ilu_.Dinv = arena_.alloc<double>(16 * nc);
     ilu_.order = arena_.alloc<int32_t>(nc);
     ilu_.sweep = arena_.alloc<int32_t>(2 * nc);
-    ilu_.lev_off = arena_.alloc<int32_t>(ilu_lev_off_h_.size());
-    ilu_.rec = arena_.alloc<int32_t>(16 * nc);
-    ilu_.out_f = arena_.alloc<Vec4<double>>(nc);
-    ilu_.out_b = arena_.alloc<Vec4<double>>(nc);
-    ilu_.pack = arena_.alloc<double>((nc + 31) / 32 * 32 * 144);
+    const SweepPlan& pl = ilu_plan_h_;
+    if (pl.cluster > 0) {
+      ilu_.cl_blocks = pl.cluster;
+      for (int d = 0; d < 2; ++d) {
+        ilu_.cl_nlev[d] = pl.nlev[d];
+        ilu_.cl_chunks[d] = (int)pl.chunks[d];
+        ilu_.cl_info[d] = arena_.alloc<int32_t>(pl.info[d].size());
+        ilu_.cl_rec[d] = arena_.alloc<int32_t>(pl.rec[d].size());
+        ilu_.pack[d] = arena_.alloc<double>(pl.chunks[d] * 2048);
+        h2d(ilu_.cl_info[d], pl.info[d], s);
+        h2d(ilu_.cl_rec[d], pl.rec[d], s);
+      }
+      ilu_.cl_pos = arena_.alloc<int32_t>(nc);
+      ilu_.packD = arena_.alloc<double>(pl.chunks[1] * 512);
+      ilu_.own_f = arena_.alloc<Vec4<double>>(pl.chunks[0] * 32);
+      ilu_.own_b = arena_.alloc<Vec4<double>>(pl.chunks[1] * 32);
+      h2d(ilu_.cl_pos, pl.pos[0], s);
+      for (auto* f : {k_ilu_sweep_cluster<true>, k_ilu_sweep_cluster<false>})
+        O2F_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem));
+    }
     ilu_.lo_cells = arena_.alloc<int32_t>(nc);
     ilu_.tmp = arena_.alloc<Vec4<double>>(nc);
     ilu_.sync = arena_.alloc<SweepSync>(2);
@@ -730,12 +711,6 @@ void Solver::ilu_factor() {
     h2d(ilu_.pos, ilu_pos_h_, s);
     h2d(ilu_.order, ilu_order_h_, s);
     h2d(ilu_.sweep, ilu_sweep_h_, s);
-    h2d(ilu_.lev_off, ilu_lev_off_h_, s);
-    h2d(ilu_.rec, ilu_rec_h_, s);
-    O2F_CUDA(cudaFuncSetAttribute(k_ilu_sweep_cta<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kSweepSmem));
-    O2F_CUDA(cudaFuncSetAttribute(k_ilu_sweep_cta<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kSweepSmem));
     h2d(ilu_.lo_cells, lo_cells_h_, s);
     k_ilu_empty<<<grid(nc), kBlock, 0, s>>>(nc, ilu_.tmp);
     O2F_CUDA(cudaMemsetAsync(ilu_.sync, 0, 2 * sizeof(SweepSync), s));
@@ -753,7 +728,10 @@ void Solver::ilu_factor() {
     k_ilu_factor<<<(n + 127) / 128, 128, 0, s>>>(ilu_.lo_cells + lo_off_h_[l], n, ilu_, ilu_status_);
   }
   // the factor blocks in the block sweeps' order
-  k_ilu_pack<<<(int)((2 * nc * 5 + 255) / 256), 256, 0, s>>>((int)nc, ilu_);
+  if (ilu_block_sweeps()) {
+    const int64_t pairs = (int64_t)ilu_.cl_chunks[0] * 1024 + (int64_t)ilu_.cl_chunks[1] * 1280;
+    k_ilu_pack<<<(int)((pairs + 255) / 256), 256, 0, s>>>(ilu_);
+  }
   O2F_CUDA(cudaGetLastError());
   launches_ += 2 + ilu_.n_lo;
   int st = 0;
@@ -762,23 +740,35 @@ void Solver::ilu_factor() {
   if (st) throw Error(O2F_ERR_BREAKDOWN, "singular block in the ILU(0) factorization");
 }
 
-// O2F_SWEEPS_AUTO: triangles up to this many rows are swept by one thread
-// block (measured on B200 per adjoint iteration alone, block / waiting:
-// 3.9 / 5.2 ms at 75k rows, 6.9 / 8.1 at 151k, 13.1 / 11.8 at 301k; side by
-// side with other contexts' solves the block sweep is ahead at every size).
-constexpr int64_t kIluCtaMaxRows = 200000;
+// O2F_SWEEPS_AUTO: block sweeps wherever they have a plan (operand slots ran
+// out on none of the O-grids up to 2.0M cells).  Measured per adjoint
+// iteration alone, block / waiting: 0.35 / 1.4 ms at 5k rows, 1.1 / 5.2 at
+// 75k, 2.3 / 11.6 at 300k, 4.5 / 20.8 at 814k.
+bool Solver::ilu_block_sweeps() const {
+  return !ilu_waiting_ && ilu_plan_h_.cluster > 0 && params_.adjoint_sweeps != O2F_SWEEPS_WAITING;
+}
 
-// z = M^{-1} r = U^{-1} L^{-1} r: the forward sweep into ilu_.tmp, the
-// backward sweep into z; one launch per triangle, either one block walking
-// the levels or persistent warps that wait on their rows' dependencies.
+// z = M^{-1} r = U^{-1} L^{-1} r, one launch per triangle: a cluster of blocks
+// walking the levels (its input is ilu_.own_f, r in forward sweep order,
+// which the vector kernels before it write), or persistent warps that wait
+// on their rows' dependencies.
 void Solver::ilu_apply(const Vec4<double>* r, Vec4<double>* z, const int* gate) {
   cudaStream_t s = stream_;
   const int n = (int)ilu_.nc;
-  const int mode = params_.adjoint_sweeps;
-  const bool block = mode == O2F_SWEEPS_BLOCK || (mode == O2F_SWEEPS_AUTO && n <= kIluCtaMaxRows);
-  if (!ilu_waiting_ && block) {  // one block per triangle, level by level
-    k_ilu_sweep_cta<true><<<1, kSweepCtaThreads, kSweepSmem, s>>>(n, ilu_, r, z, gate);
-    k_ilu_sweep_cta<false><<<1, kSweepCtaThreads, kSweepSmem, s>>>(n, ilu_, nullptr, z, gate);
+  if (ilu_block_sweeps()) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ilu_.cl_blocks);
+    cfg.blockDim = dim3(kSweepThreads);
+    cfg.dynamicSmemBytes = kSweepSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ilu_.cl_blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    O2F_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_sweep_cluster<true>, ilu_, z, gate));
+    O2F_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_sweep_cluster<false>, ilu_, z, gate));
     return;
   }
   const int blocks = ilu_sweep_blocks(n);
@@ -1412,12 +1402,15 @@ void Solver::adjoint_solve(double beta, double tol, int64_t max_iter, int64_t re
   const int kItersPerGraph = precond ? 1 : 8;
   const int kernels_per_iter = 5 + (precond ? 4 : 0);
   const int* kgate = &ks_->stop;
+  // block sweeps read their input in sweep order
+  const int32_t* spos = precond && ilu_block_sweeps() ? ilu_.cl_pos : nullptr;
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   O2F_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
   for (int i = 0; i < kItersPerGraph; ++i) {
     k_bicg_p<<<kgrid, kBlock, 0, stream_>>>(n4, reinterpret_cast<double*>(r_), reinterpret_cast<double*>(r0_),
-                                               reinterpret_cast<double*>(p_), reinterpret_cast<double*>(v_), ks_);
+                                               reinterpret_cast<double*>(p_), reinterpret_cast<double*>(v_), spos,
+                                               reinterpret_cast<double*>(ilu_.own_f), ks_);
     if (precond) ilu_apply(p_, ph, kgate);
     if (full)
       k_bicg_fjt_v<<<kgrid, kBlock, 0, stream_>>>(nc, fjac_off_, fjac_idx_, fjac_blk_, ph, v_, r0_, part_, ks_);
@@ -1428,7 +1421,8 @@ void Solver::adjoint_solve(double beta, double tol, int64_t max_iter, int64_t re
       k_bicg_jt_v<<<kgrid, kBlock, 0, stream_>>>(nc, topo_.jslot, geom_, topo_.ec, topo_.ebc, blk_, ph, v_, r0_,
                                                     part_, ks_);
     k_bicg_s<<<kgrid, kBlock, 0, stream_>>>(n4, reinterpret_cast<double*>(r_), reinterpret_cast<double*>(v_),
-                                               reinterpret_cast<double*>(s_), ks_);
+                                               reinterpret_cast<double*>(s_), spos,
+                                               reinterpret_cast<double*>(ilu_.own_f), ks_);
     if (precond) ilu_apply(s_, sh, kgate);
     if (full)
       k_bicg_fjt_t<<<kgrid, kBlock, 0, stream_>>>(nc, fjac_off_, fjac_idx_, fjac_blk_, sh, s_, t_, part_, ks_);

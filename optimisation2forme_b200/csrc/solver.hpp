@@ -13,6 +13,7 @@
 #include "device_types.hpp"
 #include "mesh_host.hpp"
 #include "o2f.h"
+#include "sweep_plan.hpp"
 
 namespace o2f {
 
@@ -197,6 +198,7 @@ class Solver {
   void ilu_factor();
   void ilu_apply(const Vec4<double>* r, Vec4<double>* z, const int* gate);
   void ilu_check_sweeps();
+  bool ilu_block_sweeps() const;  // the block sweeps, not the waiting ones
 
  public:
   void debug_ilu_stall(int stall, long long spin_limit);
@@ -204,7 +206,7 @@ class Solver {
  private:
   std::vector<int32_t> ilu_nbr_h_, ilu_pos_h_, ilu_order_h_, lo_off_h_, lo_cells_h_, ilu_sweep_h_;
   int ilu_n_up_ = 0;  // levels of the backward sweep's dependencies
-  std::vector<int32_t> ilu_lev_off_h_, ilu_rec_h_;
+  SweepPlan ilu_plan_h_;  // rows, levels and value routes of the block sweeps
   bool ilu_waiting_ = false;  // test hook: use the sweeps that wait on other rows
   IluDev ilu_{};
   bool ilu_alloc_ = false;
