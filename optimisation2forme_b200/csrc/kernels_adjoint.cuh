@@ -5,6 +5,7 @@
 #pragma once
 
 #include "kernels.cuh"
+#include "kernels_tile.cuh"
 #include "step.cuh"
 
 namespace o2f {
@@ -73,8 +74,12 @@ __device__ bool grid_reduce(double (&v)[N], double* part, unsigned int* ticket, 
 // Time-step control of Simulator::time_loop (src/simulation.cpp:68-124); the
 // per-step device functions and StepState are in step.cuh.
 
-// Start of a step: evaluate the loop condition, reset the wave-speed maximum.
-__global__ void k_step_begin(StepState* st) { step_begin_at(st); }
+// Start of a time loop: evaluate the loop condition, reset the wave-speed
+// maximum.  (Later steps are started by the tile kernels, kernels_tile.cuh.)
+__global__ void k_step_begin(StepState* st) {
+  step_begin_at(st);
+  wave_speed_reset(st);
+}
 
 // max over cells of hypot(u, v) + c (src/simulation.cpp:80-96).  The maximum
 // of positive doubles is exact, so the atomic order does not matter.
@@ -88,16 +93,22 @@ __global__ void __launch_bounds__(kBlock) k_wave_speed(int64_t nc, const Vec4<T>
   wave_speed_commit(m, st);
 }
 
-// dt = min(CFL*min_h/max_wave, 0.5*min_h^2/mu) (src/simulation.cpp:108-110).
-__global__ void k_step_dt(StepState* st) { step_dt_at(st); }
+// dt = min(CFL*min_h/max_wave, 0.5*min_h^2/mu) (src/simulation.cpp:108-110),
+// and the maximum reset for the next step.
+__global__ void k_step_dt(StepState* st) {
+  step_dt_at(st);
+  wave_speed_reset(st);
+}
 
-// Residual history: ||R_rho||_2 of the first stage, from the per-block partials.
+// After the first stage: ||R_rho||_2 of the history from the blocks' partials.
 __global__ void k_step_norm(const double* part, int nparts, double* hist, StepState* st) {
   if (st->stop) return;
   step_norm_block(part, nparts, hist, st);
 }
-
-__global__ void k_step_end(StepState* st) { step_end_at(st); }
+// After the last stage.
+__global__ void k_step_turn(StepState* st) {
+  if (!st->stop) step_turn(st);
+}
 
 // ---------------------------------------------------------------------------
 // computeLiftDragCoefficients (src/compute.cpp:92-132) and
@@ -184,8 +195,8 @@ __global__ void __launch_bounds__(128) k_jt_blocks(int64_t ne, Geom<double> g, c
       Rp = bc_ghost(code, ph, Lp);
       Rm = bc_ghost(code, ph, Lm);
     }
-    const Vec4<double> fp = hllc(Lp, Rp, eg.a, eg.b, gamma);
-    const Vec4<double> fm = hllc(Lm, Rm, eg.a, eg.b, gamma);
+    const Vec4<double> fp = hllc_flux(Lp, Rp, eg.a, eg.b, gamma);
+    const Vec4<double> fm = hllc_flux(Lm, Rm, eg.a, eg.b, gamma);
     out[0 * 4 + j] = (fp.a - fm.a) / (2 * eps);
     out[1 * 4 + j] = (fp.b - fm.b) / (2 * eps);
     out[2 * 4 + j] = (fp.c - fm.c) / (2 * eps);
@@ -202,8 +213,8 @@ __global__ void __launch_bounds__(128) k_jt_blocks(int64_t ne, Geom<double> g, c
     Vec4<double> Rp = Rs, Rm = Rs;
     comp(Rp, j) = comp(Rs, j) + eps;
     comp(Rm, j) = comp(Rs, j) - eps;
-    const Vec4<double> fp = hllc(Ls, Rp, eg.a, eg.b, gamma);
-    const Vec4<double> fm = hllc(Ls, Rm, eg.a, eg.b, gamma);
+    const Vec4<double> fp = hllc_flux(Ls, Rp, eg.a, eg.b, gamma);
+    const Vec4<double> fm = hllc_flux(Ls, Rm, eg.a, eg.b, gamma);
     out[16 + 0 * 4 + j] = (fp.a - fm.a) / (2 * eps);
     out[16 + 1 * 4 + j] = (fp.b - fm.b) / (2 * eps);
     out[16 + 2 * 4 + j] = (fp.c - fm.c) / (2 * eps);

@@ -76,7 +76,10 @@ __global__ void __launch_bounds__(kBatchMaxBlock) kb_wave_speed(const BatchItem*
 // Scalar steps: one thread per candidate.
 __global__ void kb_step_begin(const BatchItem* __restrict__ items, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) step_begin_at(items[i].st);
+  if (i < n) {
+    step_begin_at(items[i].st);
+    if (!items[i].st->stop) wave_speed_reset(items[i].st);
+  }
 }
 __global__ void kb_step_dt(const BatchItem* __restrict__ items, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -29,14 +29,22 @@ __global__ void __launch_bounds__(kBlock) k_widen(int64_t n, const float* __rest
 // writes the block partial sums of R_rho^2 in FP64.  `keep` (may be null)
 // receives the FP64 state the stage started from (the last stage's input is
 // what the FP64 path linearises about after the loop).
-template <bool kRk>
-__device__ __forceinline__ double cell_residual_mixed_at(
-    int64_t c, int64_t nc, const int32_t* __restrict__ slot, const Geom<float>& g, const Vec4<float>* __restrict__ F,
-    const Vec4<float>* __restrict__ etq, const float* __restrict__ etqy, Vec4<float>* __restrict__ U32,
+//
+// c0 uo + c1 (u + dt r), with its contraction said: left to the compiler it
+// could differ between the kernels that share this function.
+__device__ __forceinline__ double stage_update(const RkStage& rk, double uo, double u, double dt, float r) {
+  const double t = __fma_rn(dt, (double)r, u);
+  return __fma_rn(rk.c1, t, rk.c0 * uo);
+}
+
+template <bool kRk, typename ED>
+__device__ __forceinline__ double cell_residual_mixed_from(
+    int64_t c, int64_t nc, const int32_t* __restrict__ slot, const Vec4<float>* __restrict__ cgeom, ED ed,
+    Vec4<float>* __restrict__ U32,
     Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, Vec4<double>* __restrict__ R, const RkStage& rk,
-    const double* dtp, Vec4<double>* __restrict__ keep) {
+    const double* dtp, Vec4<double>* __restrict__ keep, Vec4<double>* unew = nullptr) {
   double r2 = 0.0;
-  const float cv = g.cgeom[c].c;
+  const float cv = cgeom[c].c;
   int sl[4], nk = 0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) sl[k] = slot[(int64_t)k * nc + c];
@@ -53,8 +61,9 @@ __device__ __forceinline__ double cell_residual_mixed_at(
     const int s = sl[k];
     const int e = s >> 1;
     const float sign = ((s & 1) == 0) ? 1.f : -1.f;
-    const Vec4<float> eg = g.egeom[e];
-    const Vec4<float> f = F[e];
+    const int i = ed.at(k, e);
+    const Vec4<float> eg = ed.geom(i);
+    const Vec4<float> f = ed.flux(i);
     a0 += sign * f.a * eg.c;
     a1 += sign * f.b * eg.c;
     a2 += sign * f.c * eg.c;
@@ -70,15 +79,16 @@ __device__ __forceinline__ double cell_residual_mixed_at(
     if (k >= nk) continue;
     const int s = sl[k];
     const int e = s >> 1;
-    const Vec4<float> eg = g.egeom[e];
+    const int i = ed.at(k, e);
+    const Vec4<float> eg = ed.geom(i);
     const float el = eg.c;
     float enx = eg.a, eny = eg.b;
     if ((s & 1) == 0) {
       enx = -enx;
       eny = -eny;
     }
-    const Vec4<float> t = etq[e];
-    const float qy = etqy[e];
+    const Vec4<float> t = ed.visc(i);
+    const float qy = ed.visc_y(i);
     a1 += t.a * el * enx / cv + t.c * el * eny / cv;
     a2 += t.c * el * enx / cv + t.b * el * eny / cv;
     a3 += (uu * t.a + vv * t.c - t.d) * el * enx / cv + (uu * t.c + vv * t.b - qy) * el * eny / cv;
@@ -97,14 +107,25 @@ __device__ __forceinline__ double cell_residual_mixed_at(
     } else {
       uo = Uold[c];
     }
-    u.a = rk.c0 * uo.a + rk.c1 * (u.a + dt * (double)a0);
-    u.b = rk.c0 * uo.b + rk.c1 * (u.b + dt * (double)a1);
-    u.c = rk.c0 * uo.c + rk.c1 * (u.c + dt * (double)a2);
-    u.d = rk.c0 * uo.d + rk.c1 * (u.d + dt * (double)a3);
+    u.a = stage_update(rk, uo.a, u.a, dt, a0);
+    u.b = stage_update(rk, uo.b, u.b, dt, a1);
+    u.c = stage_update(rk, uo.c, u.c, dt, a2);
+    u.d = stage_update(rk, uo.d, u.d, dt, a3);
     U[c] = u;
+    if (unew) *unew = u;
     U32[c] = v4<float>((float)u.a, (float)u.b, (float)u.c, (float)u.d);
   }
   return r2;
+}
+
+template <bool kRk>
+__device__ __forceinline__ double cell_residual_mixed_at(
+    int64_t c, int64_t nc, const int32_t* __restrict__ slot, const Geom<float>& g, const Vec4<float>* __restrict__ F,
+    const Vec4<float>* __restrict__ etq, const float* __restrict__ etqy, Vec4<float>* __restrict__ U32,
+    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, Vec4<double>* __restrict__ R, const RkStage& rk,
+    const double* dtp, Vec4<double>* __restrict__ keep) {
+  return cell_residual_mixed_from<kRk>(c, nc, slot, g.cgeom, EdgeFluxes<float>{g.egeom, F, etq, etqy}, U32, U, Uold, R,
+                                       rk, dtp, keep);
 }
 
 template <bool kRk>

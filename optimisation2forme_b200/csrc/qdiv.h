@@ -75,6 +75,87 @@ O2F_QDIV_FN double qdiv_flag(double a, double b, double y, bool& ok) {
   return fma(r1, y, q1);
 }
 
+// Without branches, for code that keeps many quotients in flight: the
+// reciprocal comes from a seed by Newton's iteration and Markstein's final
+// correction, and whatever leaves the range of the proofs above clears `ok`
+// (the caller then recomputes with plain division).
+//
+// recip_seeded: y0 within 2^-18 of 1/b (relative).  Two Newton steps leave an
+// error below one ulp, and RN(y + y * RN(1 - b*y)) is then RN(1/b) unless b's
+// significand is all ones (Markstein 1990; Muller et al., ch. 4), which is
+// excluded here.
+O2F_QDIV_FN unsigned high_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return (unsigned)__double2hiint(x);
+#else
+  unsigned long long u;
+  __builtin_memcpy(&u, &x, 8);
+  return (unsigned)(u >> 32);
+#endif
+}
+O2F_QDIV_FN unsigned low_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return (unsigned)__double2loint(x);
+#else
+  unsigned long long u;
+  __builtin_memcpy(&u, &x, 8);
+  return (unsigned)u;
+#endif
+}
+// 2^-400 <= |x| < 2^400, by the exponent field.
+O2F_QDIV_FN bool mid_range(double x) { return (high_word(x) & 0x7fffffffu) - 0x26f00000u < 0x32000000u; }
+O2F_QDIV_FN bool is_zero(double x) { return ((high_word(x) & 0x7fffffffu) | low_word(x)) == 0u; }
+
+O2F_QDIV_FN double recip_seeded(double b, double y0, bool& ok) {
+  ok &= mid_range(b) & !(((high_word(b) & 0xfffffu) == 0xfffffu) & (low_word(b) == 0xffffffffu));
+  const double y1 = fma(y0, fma(-b, y0, 1.0), y0);
+  const double y2 = fma(y1, fma(-b, y1, 1.0), y1);
+  return fma(y2, fma(-b, y2, 1.0), y2);
+}
+
+// RN(a/b) given y = RN(1/b); zero numerators included (with the quotient's sign).
+O2F_QDIV_FN double quot(double a, double b, double y, bool& ok) {
+  const double q0 = a * y;
+  const bool zero = is_zero(a);
+  ok &= mid_range(q0) | zero;
+  const double r0 = fma(-b, q0, a);
+  const double q1 = fma(r0, y, q0);
+  const double r1 = fma(-b, q1, a);
+  const double q = fma(r1, y, q1);
+  return zero ? q0 : q;
+}
+
+// RN(sqrt(a)) for a > 0 from a seed y0 within 2^-18 of 1/sqrt(a) (relative):
+// Goldschmidt's iteration on g = sqrt(a), h = 1/(2 sqrt(a)), then Markstein's
+// correction g + h (a - g g), whose residual is exact (Muller et al., ch. 4).
+O2F_QDIV_FN double sqrt_seeded(double a, double y0, bool& ok) {
+  ok &= mid_range(a) & (high_word(a) < 0x80000000u);
+  double g = a * y0, h = 0.5 * y0;
+  double r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  r = fma(-g, h, 0.5);
+  g = fma(g, r, g);
+  h = fma(h, r, h);
+  g = fma(h, fma(-g, g, a), g);
+  return fma(h, fma(-g, g, a), g);
+}
+
+#if defined(__CUDACC__)
+__device__ __forceinline__ double sqrt_fast(double a, bool& ok) {
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
+  return sqrt_seeded(a, y0, ok);
+}
+__device__ __forceinline__ double recip_fast(double b, bool& ok) {
+  double y0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
+  return recip_seeded(b, y0, ok);
+}
+__device__ __forceinline__ float recip_fast(float b, bool&) { return 1.0f / b; }
+__device__ __forceinline__ float quot(float a, float, float y, bool&) { return a * y; }
+#endif
+
 // FP32 instantiations (the mixed-precision path, which is not bit-exact by
 // design): one reciprocal per divisor, each quotient a multiplication
 // (within 1.5 ulp of a/b).

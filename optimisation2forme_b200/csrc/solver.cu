@@ -62,6 +62,15 @@ void validate_params(const o2f_params& p) {
   if (!(p.adjoint_shift >= 0.0) || !(p.adjoint_shift < 1e6)) throw Error(O2F_ERR_ARG, "adjoint_shift out of range");
 }
 
+// Cells per tile of the time loop's kernels (= threads per block), 0: the
+// separate kernels.  Up to here a step is bound by the latency of its
+// kernels, beyond it by their throughput, where the separate kernels run
+// with more warps.  Measured, us per FP64 step, tiles of 128 / separate:
+// 62 / 80 at 3,840 triangles, 80 / 105 at 74,528, 159 / 193 at 150,544,
+// 230 / 233 at 213,440, 344 / 320 at 300,300; tiles of 64 and 96 cells are
+// behind 128 at every size.  (FP32: 46 / 68, 60 / 84, 113 / 113, 154 / 133.)
+int tile_cells(int64_t nc) { return nc < 180000 ? kTileMax : 0; }
+
 }  // namespace
 
 Solver::Solver(const o2f_mesh_desc& desc, const o2f_params& p, cudaStream_t stream) {
@@ -324,7 +333,6 @@ void Solver::upload_mesh() {
   work_ = alloc_work();
   U_ = arena_.alloc<Vec4<double>>(nc);
   Uold_ = arena_.alloc<Vec4<double>>(nc);
-  norm_part_ = arena_.alloc<double>(grid(nc));
   step_ = arena_.alloc<StepState>(1);
   part_ = arena_.alloc<double>(kRedGrid * 4);
   ticket_ = arena_.alloc<unsigned int>(4);
@@ -334,6 +342,8 @@ void Solver::upload_mesh() {
   O2F_CUDA(cudaMemsetAsync(ks_, 0, sizeof(KrylovState), s));
   sync();  // host staging vectors go out of scope
   setup_ilu_host(jslot, ec, ebc);
+  slot_h_ = std::move(slot);
+  ev_h_ = std::move(ev);
 }
 
 // Geometry of the host mesh in device order: cell centres and volumes, edge
@@ -894,10 +904,10 @@ void Solver::launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<
     k_cell_gradient_alpha<2><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_, w.eL,
                                                             w.eR, w.ctq, w.ctqy, fjac_alpha_);
   else if (write_grad)
-    k_cell_gradient<double, true><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_,
+    k_cell_gradient<double, true><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_,
                                                                 w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
   else
-    k_cell_gradient<double, false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_,
+    k_cell_gradient<double, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_,
                                                                  w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
   k_vertex_visc<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq,
                                                       w.vtqy, gate);
@@ -969,7 +979,7 @@ void Solver::profile_kernels(int reps, double* ms_out) {
                                                                nullptr);
           break;
         case O2F_K_CELL_GRADIENT:
-          k_cell_gradient<double, false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U_, w.vq,
+          k_cell_gradient<double, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U_, w.vq,
                                                                        phys_, w.eL, w.eR, w.ctq, w.ctqy, w.grad,
                                                                        nullptr);
           break;
@@ -1057,6 +1067,138 @@ void Solver::debug_get(const std::string& which, double* out) {
   }
 }
 
+// Tiles of consecutive cells with their vertices and edges, for meshes whose
+// time loop runs on them.
+void Solver::build_tiles() {
+  const int64_t nc = topo_.nc;
+  if (!norm_part_) norm_part_ = arena_.alloc<double>(grid(nc) * (kBlock / kTileMax));
+  const int T = tile_cells(nc);
+  if (tiles_ || T == 0) return;
+  const int nt = (int)((nc + T - 1) / T);
+  TileDev td{};
+  td.n = nt;
+  td.cells = T;
+  std::vector<int32_t> voff(nt + 1, 0), eoff(nt + 1, 0), verts, edges;
+  std::vector<ushort2> cell_v(4 * nc, ushort2{0, 0}), edge_v;
+  std::vector<uint16_t> cell_e(4 * nc, 0);
+  verts.reserve(topo_.nv * 3 / 2);
+  edges.reserve(topo_.ne * 5 / 4);
+  edge_v.reserve(topo_.ne * 5 / 4);
+  // tile that listed an entity last, and its place in that list
+  std::vector<int32_t> vt(topo_.nv, -1), et(topo_.ne, -1), vi(topo_.nv), ei(topo_.ne);
+  for (int b = 0; b < nt; ++b) {
+    const int64_t c0 = (int64_t)b * T, c1 = std::min(nc, c0 + T);
+    for (int64_t c = c0; c < c1; ++c)
+      for (int k = 0; k < 4; ++k) {
+        const int32_t s = slot_h_[k * nc + c];
+        if (s < 0) continue;
+        const int32_t e = s >> 1;
+        if (et[e] == b) continue;
+        et[e] = b;
+        edges.push_back(e);
+        for (int32_t v : {ev_h_[e].x, ev_h_[e].y})
+          if (vt[v] != b) {
+            vt[v] = b;
+            verts.push_back(v);
+          }
+      }
+    std::sort(verts.begin() + voff[b], verts.end());
+    std::sort(edges.begin() + eoff[b], edges.end());
+    voff[b + 1] = (int32_t)verts.size();
+    eoff[b + 1] = (int32_t)edges.size();
+    for (int32_t i = voff[b]; i < voff[b + 1]; ++i) vi[verts[i]] = i - voff[b];
+    for (int32_t i = eoff[b]; i < eoff[b + 1]; ++i) {
+      ei[edges[i]] = i - eoff[b];
+      const int2 x = ev_h_[edges[i]];
+      edge_v.push_back(ushort2{(unsigned short)vi[x.x], (unsigned short)vi[x.y]});
+    }
+    for (int64_t c = c0; c < c1; ++c)
+      for (int k = 0; k < 4; ++k) {
+        const int32_t s = slot_h_[k * nc + c];
+        if (s < 0) continue;
+        const int2 x = ev_h_[s >> 1];
+        cell_e[k * nc + c] = (uint16_t)ei[s >> 1];
+        cell_v[k * nc + c] = ushort2{(unsigned short)vi[x.x], (unsigned short)vi[x.y]};
+      }
+    td.max_verts = std::max(td.max_verts, voff[b + 1] - voff[b]);
+    td.max_edges = std::max(td.max_edges, eoff[b + 1] - eoff[b]);
+  }
+  auto up = [&](const auto& h) {
+    auto* d = arena_.alloc<std::decay_t<decltype(h[0])>>(h.size());
+    h2d(d, h, stream_);
+    return d;
+  };
+  td.voff = up(voff);
+  td.verts = up(verts);
+  td.eoff = up(eoff);
+  td.edges = up(edges);
+  td.edge_v = up(edge_v);
+  td.cell_v = up(cell_v);
+  td.cell_e = up(cell_e);
+  sync();
+  tiles_ = std::make_unique<TileDev>(td);
+  slot_h_ = {};
+  ev_h_ = {};
+  // (one value for every mesh: contexts of other threads may be launching)
+  for (auto* f : {k_tile_residual<1>, k_tile_residual<2>, k_tile_residual<3>})
+    O2F_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax));
+  tile_smem_f32();
+}
+
+// Step control of the separate kernels.
+void Solver::step_control(int stage) {
+  if (stage == 1) k_step_norm<<<1, 1024, 0, stream_>>>(norm_part_, grid(topo_.nc), hist_dev_, step_);
+  if (stage == 3) k_step_turn<<<1, 1, 0, stream_>>>(step_);
+}
+
+void Solver::launch_stage(int stage, const RkStage& rk) {
+  cudaStream_t s = stream_;
+  if (!tiles_) {
+    const Topo& t = topo_;
+    const Geom<double>& g = geom_;
+    const Work<double>& w = work_;
+    const int* gate = &step_->stop;
+    k_vertex_state<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U_, phys_, w.vq, gate);
+    k_cell_gradient<double, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(
+        t.nc, t.slot, g, t.ev, t.ec, t.ebc, U_, w.vq, phys_, w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
+    k_vertex_visc<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
+                                                        gate);
+    k_edge_flux<double><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F,
+                                                      w.etq, w.etqy, gate);
+    auto* last = stage == 1 ? k_cell_residual_stage<1> : stage == 2 ? k_cell_residual_stage<2> : k_cell_residual_stage<3>;
+    last<<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, phys_, w, U_, Uold_, rk, norm_part_, step_);
+    step_control(stage);
+    O2F_CUDA(cudaGetLastError());
+    return;
+  }
+  const TileDev& td = *tiles_;
+  // the last stage leaves its vertex states, as a residual does
+  O2F_CUDA(tile_launch(k_tile_gradient<double>, td, tile_gradient_smem<double>(td), s, td, topo_, geom_, U_, phys_, work_,
+                       stage == 3 ? work_.vq : nullptr, &step_->stop));
+  auto* last = stage == 1 ? k_tile_residual<1> : stage == 2 ? k_tile_residual<2> : k_tile_residual<3>;
+  O2F_CUDA(tile_launch(last, td, tile_residual_smem<double>(td), s, td, topo_, geom_, phys_, work_, U_, Uold_, rk,
+                       norm_part_, hist_dev_, step_));
+}
+
+// What a residual leaves in the context beyond the interface states: vertex
+// viscous quantities, fluxes and edge viscous quantities (wall stresses) of
+// the loop's last residual, and its vertex states when the loop stopped in a
+// first stage (its input is then U_old).
+void Solver::publish_stage(bool first_stage) {
+  const Topo& t = topo_;
+  const Geom<double>& g = geom_;
+  const Work<double>& w = work_;
+  cudaStream_t s = stream_;
+  if (first_stage)
+    k_vertex_state<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, Uold_, phys_, w.vq, nullptr);
+  k_vertex_visc<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
+                                                      nullptr);
+  k_edge_flux<double><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F, w.etq,
+                                                    w.etqy, nullptr);
+  O2F_CUDA(cudaGetLastError());
+  launches_ += first_stage ? 3 : 2;
+}
+
 void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_t* steps_done, double* t_out) {
   NvtxRange nvtx_("o2f rk3_run");
   if (max_steps < 0) throw Error(O2F_ERR_ARG, "max_steps < 0");
@@ -1075,12 +1217,11 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
   st.drop_tol = drop_tol;
   st.max_steps = max_steps;
   O2F_CUDA(cudaMemcpyAsync(step_, &st, sizeof(st), cudaMemcpyHostToDevice, stream_));
-  const int* gate = &step_->stop;
+  build_tiles();
   const double* dt = &step_->dt;
   const RkStage s1{0.0, 1.0, dt, 1, norm_part_};
   const RkStage s2{3.0 / 4.0, 1.0 / 4.0, dt, 0, nullptr};
   const RkStage s3{1.0 / 3.0, 2.0 / 3.0, dt, 0, nullptr};
-  const int nparts = grid(topo_.nc);
   const int wave_grid = std::min(grid(topo_.nc), 148 * 8);
   // One CUDA graph holds kStepsPerGraph steps; steps past a stop condition
   // are no-ops (every kernel checks the gate).
@@ -1092,24 +1233,25 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
     ensure_f32();
     f32_state_sync();
   }
-  auto stage = [&](const RkStage* rk) {
+  auto stage = [&](int k, const RkStage& rk) {
     if (mixed)
-      launch_residual_f32(gate, rk, rk == &s3 ? Ukeep_ : nullptr);
+      launch_stage_f32(k, rk);
     else
-      launch_residual(geom_, work_, U_, gate, false, rk);
+      launch_stage(k, rk);
   };
+  // the first step's dt; every later one is set at the end of the step before
+  k_step_begin<<<1, 1, 0, stream_>>>(step_);
+  k_wave_speed<double><<<wave_grid, kBlock, 0, stream_>>>(topo_.nc, U_, params_.gamma, step_);
+  k_step_dt<<<1, 1, 0, stream_>>>(step_);
+  O2F_CUDA(cudaGetLastError());
+  launches_ += 3;
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   O2F_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
   for (int i = 0; i < kStepsPerGraph; ++i) {
-    k_step_begin<<<1, 1, 0, stream_>>>(step_);
-    k_wave_speed<double><<<wave_grid, kBlock, 0, stream_>>>(topo_.nc, U_, params_.gamma, step_);
-    k_step_dt<<<1, 1, 0, stream_>>>(step_);
-    stage(&s1);
-    k_step_norm<<<1, 1024, 0, stream_>>>(norm_part_, nparts, hist_dev_, step_);
-    stage(&s2);
-    stage(&s3);
-    k_step_end<<<1, 1, 0, stream_>>>(step_);
+    stage(1, s1);
+    stage(2, s2);
+    stage(3, s3);
   }
   O2F_CUDA(cudaStreamEndCapture(stream_, &graph));
   O2F_CUDA(cudaGraphInstantiate(&exec, graph, 0));
@@ -1119,7 +1261,7 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
     while (true) {
       O2F_CUDA(cudaGraphLaunch(exec, stream_));
       launched += kStepsPerGraph;
-      launches_ += kStepsPerGraph * 20;
+      launches_ += kStepsPerGraph * (tiles_ ? 6 : 17);
       if (launched % (kStepsPerGraph * 4) == 0 || launched >= max_steps) {
         O2F_CUDA(cudaMemcpyAsync(host_st, step_, sizeof(StepState), cudaMemcpyDeviceToHost, stream_));
         sync();
@@ -1146,6 +1288,7 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
     launch_residual(geom_, work_, Ukeep_, nullptr, false, nullptr);
     sync();
   }
+  if (!mixed && tiles_ && (fin.step > 0 || fin.stop == 2)) publish_stage(fin.stop == 2);
   have_residual_ = fin.step > 0;
   invalidate_linearisation();
   if (fin.stop == 2) throw Error(O2F_ERR_NONFINITE, "non-finite state or residual in the time loop");

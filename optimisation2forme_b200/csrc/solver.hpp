@@ -19,6 +19,8 @@ namespace o2f {
 
 struct KrylovState;
 struct StepState;
+struct TileDev;
+struct RkStage;
 
 // NVTX range over a host stage (residual, time loop, adjoint, gradient,
 // Jacobian builds, mesh updates, images): named spans for Nsight tools; a
@@ -125,6 +127,13 @@ class Solver {
   // (the frozen-limiter linearisation); 0 everywhere else.
   void launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, const int* gate,
                        bool write_grad, const void* rk, int alpha_mode = 0);
+  // One RK3 stage of the time loop (kernels_tile.cuh).
+  void launch_stage(int stage, const RkStage& rk);
+  void launch_stage_f32(int stage, const RkStage& rk);
+  void step_control(int stage);
+  void build_tiles();
+  void tile_smem_f32();
+  void publish_stage(bool first_stage);
   void build_jt_blocks();
   // Both linearisations (first-order blocks, full Jacobian) belong to the
   // state, geometry and parameters they were built for.
@@ -155,6 +164,7 @@ class Solver {
   void to_reference(const Vec4<double>* dev, double* ref);
   void sync();
   int grid(int64_t n) const { return (int)((n + 255) / 256); }
+  int grad_grid(int64_t n) const { return (int)((n + 127) / 128); }  // k_cell_gradient's blocks of 128
 
   cudaStream_t stream_ = nullptr;
   bool own_stream_ = false;
@@ -178,6 +188,9 @@ class Solver {
   Vec4<double>* Ukeep_ = nullptr;  // mixed path: input state of the last RK3 stage
   float* blk32_ = nullptr;
   double* norm_part_ = nullptr;
+  std::unique_ptr<TileDev> tiles_;  // tiles of the time loop's kernels
+  std::vector<int32_t> slot_h_;     // host copies for them, until they are built
+  std::vector<int2> ev_h_;
   StepState* step_ = nullptr;
   double* hist_dev_ = nullptr;
   int64_t hist_cap_ = 0;

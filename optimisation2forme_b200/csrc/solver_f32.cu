@@ -11,6 +11,7 @@
 #include "batch.hpp"
 #include "batch_device.cuh"
 #include "kernels_f32.cuh"
+#include "kernels_tile.cuh"
 #include "solver.hpp"
 #include "step.cuh"
 
@@ -91,6 +92,45 @@ void batch_launch_mixed(int phase, bool rk, const RkStage& stage, bool keep, con
   }
 }
 
+// FP32 residual, update of the FP64 state and its FP32 shadow.
+template <int kStage>
+__global__ void __launch_bounds__(kTileMax, 4) k_tile_residual_mixed(
+    TileDev td, Topo t, Geom<float> g, Phys ph, Work<float> w, Vec4<float>* __restrict__ U32,
+    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, RkStage rk, Vec4<double>* __restrict__ keep,
+    double* part, double* hist, StepState* st) {
+  extern __shared__ __align__(32) unsigned char tile_sm[];
+  const int64_t c = (int64_t)blockIdx.x * td.cells + threadIdx.x;
+  const bool mine = threadIdx.x < td.cells && c < t.nc;
+  TileFluxes<float> ed;
+  if (!tile_fluxes<float>(blockIdx.x, td, t, g, ph, w, c, tile_sm, &st->stop, ed)) return;
+  double r2 = 0.0, wave = 0.0;
+  if (mine) {
+    Vec4<double> u;
+    r2 = cell_residual_mixed_from<true>(c, t.nc, t.slot, g.cgeom, ed, U32, U, Uold, nullptr, rk, rk.dt, keep, &u);
+    if (kStage == 3) wave_speed_cell(u, ph.gamma, wave);
+  }
+  stage_sums<kStage>(r2, wave, part, st);
+  if (kStage != 2) tile_stage_end<kStage>(td.n, part, hist, st);
+}
+
+// The cell phase of the separate kernels in the time loop.
+template <int kStage>
+__global__ void __launch_bounds__(kBlock) k_cell_residual_mixed_stage(
+    int64_t nc, const int32_t* __restrict__ slot, Geom<float> g, Phys ph, Work<float> w, Vec4<float>* __restrict__ U32,
+    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, RkStage rk, Vec4<double>* __restrict__ keep,
+    double* part, StepState* st) {
+  if (gated(&st->stop)) return;
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  double r2 = 0.0, wave = 0.0;
+  if (c < nc) {
+    Vec4<double> u;
+    r2 = cell_residual_mixed_from<true>(c, nc, slot, g.cgeom, EdgeFluxes<float>{g.egeom, w.F, w.etq, w.etqy}, U32, U,
+                                        Uold, nullptr, rk, rk.dt, keep, &u);
+    if (kStage == 3) wave_speed_cell(u, ph.gamma, wave);
+  }
+  stage_sums<kStage>(r2, wave, part, st);
+}
+
 namespace {
 int grid_of(int64_t n) { return (int)std::min<int64_t>((n + kBlock - 1) / kBlock, 148 * 16); }
 
@@ -169,7 +209,7 @@ void Solver::launch_residual_f32(const int* gate, const void* rkp, Vec4<double>*
   const Work<float>& w = work32_;
   cudaStream_t s = stream_;
   k_vertex_state<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U32_, phys_, w.vq, gate);
-  k_cell_gradient<float, false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
+  k_cell_gradient<float, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
                                                               w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
   k_vertex_visc<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
                                                      gate);
@@ -187,6 +227,47 @@ void Solver::launch_residual_f32(const int* gate, const void* rkp, Vec4<double>*
   O2F_CUDA(cudaGetLastError());
 }
 
+// Shared memory above the default for the FP32 tile kernels.
+void Solver::tile_smem_f32() {
+  for (auto* f : {k_tile_residual_mixed<1>, k_tile_residual_mixed<2>, k_tile_residual_mixed<3>})
+    O2F_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax));
+}
+
+// One RK3 stage of the time loop.
+void Solver::launch_stage_f32(int stage, const RkStage& rk) {
+  const Topo& t = topo_;
+  const Geom<float>& g = geom32_;
+  const Work<float>& w = work32_;
+  cudaStream_t s = stream_;
+  StepState* st = step_;
+  if (tiles_) {
+    const TileDev& td = *tiles_;
+    O2F_CUDA(tile_launch(k_tile_gradient<float>, td, tile_gradient_smem<float>(td), s, td, t, g, U32_, phys_, w, nullptr,
+                         &st->stop));
+    auto* last = stage == 1   ? k_tile_residual_mixed<1>
+                 : stage == 2 ? k_tile_residual_mixed<2>
+                              : k_tile_residual_mixed<3>;
+    O2F_CUDA(tile_launch(last, td, tile_residual_smem<float>(td), s, td, t, g, phys_, w, U32_, U_, Uold_, rk,
+                         stage == 3 ? Ukeep_ : nullptr, norm_part_, hist_dev_, st));
+    return;
+  }
+  const int* gate = &st->stop;
+  k_vertex_state<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U32_, phys_, w.vq, gate);
+  k_cell_gradient<float, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
+                                                             w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
+  k_vertex_visc<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
+                                                     gate);
+  k_edge_flux<float><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F, w.etq,
+                                                   w.etqy, gate);
+  auto* last = stage == 1   ? k_cell_residual_mixed_stage<1>
+               : stage == 2 ? k_cell_residual_mixed_stage<2>
+                            : k_cell_residual_mixed_stage<3>;
+  last<<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, phys_, w, U32_, U_, Uold_, rk, stage == 3 ? Ukeep_ : nullptr,
+                                     norm_part_, st);
+  step_control(stage);
+  O2F_CUDA(cudaGetLastError());
+}
+
 void Solver::profile_kernel_f32(int k) {
   const Topo& t = topo_;
   const Geom<float>& g = geom32_;
@@ -197,7 +278,7 @@ void Solver::profile_kernel_f32(int k) {
       k_vertex_state<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U32_, phys_, w.vq, nullptr);
       break;
     case O2F_K_CELL_GRADIENT:
-      k_cell_gradient<float, false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
+      k_cell_gradient<float, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
                                                                   w.eL, w.eR, w.ctq, w.ctqy, w.grad, nullptr);
       break;
     case O2F_K_VERTEX_VISC:

@@ -14,15 +14,16 @@ struct StepState {
   long long step, max_steps;
   int stop;  // 0 running, 1 finished (time, step cap or residual drop), 2 non-finite
   int drop_hit;
+  unsigned int ticket;  // blocks of a tile kernel that have ended (kernels_tile.cuh)
+  int pad;
 };
 
-// Start of a step: evaluate the loop condition, reset the wave-speed maximum.
+// Start of a step: evaluate the loop condition.
 __device__ __forceinline__ void step_begin_at(StepState* st) {
   if (st->stop) return;
-  if (!(st->t < st->final_time) || st->step >= st->max_steps || st->drop_hit) {
-    st->stop = 1;
-    return;
-  }
+  if (!(st->t < st->final_time) || st->step >= st->max_steps || st->drop_hit) st->stop = 1;
+}
+__device__ __forceinline__ void wave_speed_reset(StepState* st) {
   st->max_wave_bits = (unsigned long long)__double_as_longlong(1e-8);
 }
 // |u| + c of one cell state folded into the running maximum m with the
@@ -34,10 +35,12 @@ template <typename T>
 __device__ __forceinline__ void wave_speed_cell(const Vec4<T>& q, double gamma, double& m) {
   const double rho = q.a, ru = q.b, rv = q.c, E = q.d;
   const double u = ru / rho, v = rv / rho;
-  const double kinetic = 0.5 * (ru * ru + rv * rv) / rho;
-  const double p = (gamma - 1.0) * (E - kinetic);
-  const double cs = sqrt(gamma * p / rho);
-  const double speed = hypot(u, v) + cs;
+  // (never contracted: the FP32 loop's kernels, whose translation unit is
+  // compiled with contraction, take the same dt as the others)
+  const double kinetic = 0.5 * __dadd_rn(__dmul_rn(ru, ru), __dmul_rn(rv, rv)) / rho;
+  const double p = __dmul_rn(gamma - 1.0, __dadd_rn(E, -kinetic));
+  const double cs = sqrt(__dmul_rn(gamma, p) / rho);
+  const double speed = __dadd_rn(hypot(u, v), cs);
   if (speed > m) m = speed;
 }
 
@@ -59,11 +62,20 @@ __device__ __forceinline__ void step_dt_at(StepState* st) {
   const double dt_diff = 0.5 * (st->min_h * st->min_h) / st->mu;
   st->dt = smin(dt_adv, dt_diff);
 }
+// The same for the next step, with the maximum reset for the one after.
+__device__ __forceinline__ void step_dt_next(StepState* st) {
+  // the maximum was gathered by other blocks of this kernel: past L1
+  st->max_wave_bits = atomicMax(&st->max_wave_bits, 0ull);
+  step_dt_at(st);
+  wave_speed_reset(st);
+}
 // One block: fold the partials, record the norm and the stop conditions.
+// kFresh: they were written by other blocks of this kernel (read past L1).
+template <bool kFresh = false>
 __device__ __forceinline__ void step_norm_block(const double* part, int nparts, double* hist, StepState* st) {
   __shared__ double sm[32];
   double s = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += part[i];
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += kFresh ? __ldcg(part + i) : part[i];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   __syncthreads();
