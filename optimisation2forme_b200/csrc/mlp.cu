@@ -17,40 +17,56 @@
 namespace o2f {
 namespace mlp {
 
+// Layers as k_adam sees them: where a layer's weights start, end, and go.
+struct Layers {
+  int64_t w_off[5], w_end[5];
+  int cols[5], rows[5];
+  bf16 *W[5], *WT[5];
+};
+
 namespace {
 
 constexpr int kIn = 7;         // x, y, m, p, t, Mach, AoA
 constexpr int kFreq = 32;      // Fourier frequencies of (x, y)
 constexpr int kFeat = 128;     // 2*kFreq sin/cos + kIn raw inputs, zero padded
 constexpr int kWidth = 256;
-constexpr int kHidden = 4;
+constexpr int kHidden = 4;     // Layers holds kHidden + 1
 constexpr int kOut = 8;
 constexpr int kOutPad = 16;    // the output layer's GEMM tile width
-constexpr int kSmemBytes = 100 * 1024;  // also caps residency at 2 CTAs (2 x 256 TMEM columns) per SM
 
 int in_dim(int l) { return l == 0 ? kFeat : kWidth; }
 int out_dim(int l) { return l == kHidden ? kOutPad : kWidth; }
 
+// What a training step reads besides the data: Adam's bias corrections, the
+// step's number (place of its loss), the rows of its batch.
+struct StepHead {
+  float c1, c2;
+  int step, pad;
+};
+
+// 32 threads per row: one frequency each, and the raw inputs and the padding.
 __global__ void k_features(int n, const float* __restrict__ inputs, const int* __restrict__ index,
                            const float* __restrict__ freq, bf16* __restrict__ X) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(t >> 5), f = (int)(t & 31);
   if (i >= n) return;
   const float* in = inputs + (int64_t)(index ? index[i] : i) * kIn;
   bf16* x = X + (int64_t)i * kFeat;
   const float px = in[0], py = in[1];
-  for (int f = 0; f < kFreq; ++f) {
-    const float arg = 6.283185307179586f * (freq[2 * f] * px + freq[2 * f + 1] * py);
-    x[f] = __float2bfloat16_rn(sinf(arg));
-    x[kFreq + f] = __float2bfloat16_rn(cosf(arg));
-  }
-  for (int j = 0; j < kIn; ++j) x[2 * kFreq + j] = __float2bfloat16_rn(in[j]);
-  for (int j = 2 * kFreq + kIn; j < kFeat; ++j) x[j] = __float2bfloat16_rn(0.f);
+  const float arg = 6.283185307179586f * (freq[2 * f] * px + freq[2 * f + 1] * py);
+  x[f] = __float2bfloat16_rn(sinf(arg));
+  x[kFreq + f] = __float2bfloat16_rn(cosf(arg));
+  x[2 * kFreq + f] = __float2bfloat16_rn(f < kIn ? in[f] : 0.f);
+  x[3 * kFreq + f] = __float2bfloat16_rn(0.f);
 }
+static_assert(kFreq == 32 && kFeat == 4 * kFreq, "k_features' thread layout");
 
 // Mean squared error over the 8 outputs; dY = d(loss)/dY (bf16, padded
 // columns zero); loss accumulated into *loss.
 __global__ void k_loss(int n, const float* __restrict__ Y, const float* __restrict__ targets,
-                       const int* __restrict__ index, bf16* __restrict__ dY, float* loss) {
+                       const int* __restrict__ index, bf16* __restrict__ dY, float* loss,
+                       const StepHead* head) {
+  if (head) loss += head->step;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   float l = 0.f;
   if (i < n) {
@@ -70,29 +86,29 @@ __global__ void k_loss(int n, const float* __restrict__ Y, const float* __restri
   if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, l / ((float)n * kOut));
 }
 
-// db[j] += sum over rows of G(row, j)
-__global__ void k_colsum(int n, int cols, const bf16* __restrict__ G, float* __restrict__ db) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= cols) return;
-  const int rows_per = (n + gridDim.y - 1) / gridDim.y;
-  const int r0 = blockIdx.y * rows_per, r1 = min(n, r0 + rows_per);
-  float s = 0.f;
-  for (int r = r0; r < r1; ++r) s += __bfloat162float(G[(int64_t)r * cols + j]);
-  atomicAdd(db + j, s);
-}
-
-// Adam on the FP32 master parameters, then the BF16 copies of the weights in
+// Adam on the FP32 master parameters, and the BF16 copies of the weights in
 // both orientations (W: [out][in] for the forward GEMM, WT: [in][out] for the
 // input gradients).
 __global__ void k_adam(int64_t n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2) {
+                       float* __restrict__ v, float lr, float b1, float b2, float eps, const StepHead* head,
+                       Layers ly) {
+  const float c1 = head->c1, c2 = head->c2;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
     const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[i] = wi;
+#pragma unroll
+    for (int l = 0; l <= kHidden; ++l)
+      if (i >= ly.w_off[l] && i < ly.w_end[l]) {
+        const int j = (int)(i - ly.w_off[l]), r = j / ly.cols[l], c = j - r * ly.cols[l];
+        const bf16 b = __float2bfloat16_rn(wi);
+        ly.W[l][j] = b;
+        ly.WT[l][(int64_t)c * ly.rows[l] + r] = b;
+      }
   }
 }
 
@@ -113,8 +129,12 @@ Mlp::Mlp(int max_batch, float freq_scale, uint64_t seed, cudaStream_t stream)
     : max_batch_(max_batch), stream_(stream) {
   if (max_batch < 128 || max_batch > (1 << 20)) throw Error(O2F_ERR_ARG, "max_batch out of range [128, 2^20]");
   if (!(freq_scale > 0.f)) throw Error(O2F_ERR_ARG, "freq_scale must be positive");
-  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                gemm_smem_bytes<64>()));
+  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                gemm_smem_bytes<64>()));
+  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                gemm_smem_bytes<16>()));
   // parameter layout: W0, b0, W1, b1, ..., W4, b4
   int64_t off = 0;
   for (int l = 0; l <= kHidden; ++l) {
@@ -144,16 +164,16 @@ Mlp::Mlp(int max_batch, float freq_scale, uint64_t seed, cudaStream_t stream)
     Wb_[l] = arena_.alloc<bf16>(n);
     WTb_[l] = arena_.alloc<bf16>(n);
   }
-  X0_ = arena_.alloc<bf16>((int64_t)max_batch * kFeat);
-  for (int l = 0; l < kHidden; ++l) {
-    Z_[l] = arena_.alloc<bf16>((int64_t)max_batch * kWidth);
-    A_[l] = arena_.alloc<bf16>((int64_t)max_batch * kWidth);
-  }
+  // activations, pre-activations and their gradients of every layer: one block
+  bf16* act = arena_.alloc<bf16>((int64_t)max_batch * (kFeat + 3 * kHidden * kWidth));
+  X0_ = act;
+  act += (int64_t)max_batch * kFeat;
+  for (auto* group : {Z_, A_, dZ_})
+    for (int l = 0; l < kHidden; ++l, act += (int64_t)max_batch * kWidth) group[l] = act;
   Y_ = arena_.alloc<float>((int64_t)max_batch * kOutPad);
   dY_ = arena_.alloc<bf16>((int64_t)max_batch * kOutPad);
-  dZa_ = arena_.alloc<bf16>((int64_t)max_batch * kWidth);
-  dZb_ = arena_.alloc<bf16>((int64_t)max_batch * kWidth);
-  index_ = arena_.alloc<int>(max_batch);
+  static_assert(sizeof(StepHead) % sizeof(int) == 0, "head and indices in one buffer");
+  step_in_ = arena_.alloc<int>(sizeof(StepHead) / sizeof(int) + max_batch);
   loss_ = arena_.alloc<float>(1);
   err_ = arena_.alloc<int>(1);
   O2F_CUDA(cudaMemcpyAsync(params_, p.data(), n_params_ * sizeof(float), cudaMemcpyHostToDevice, stream_));
@@ -183,14 +203,20 @@ void Mlp::pack() {
   O2F_CUDA(cudaGetLastError());
 }
 
-void Mlp::gemm(int nt, const GemmArgs& a, int splits) {
-  const dim3 grid(blocks_of(a.M, kTileM), blocks_of(a.N, nt), splits);
-  if (nt == 256)
-    k_gemm_tc<256><<<grid, kGemmThreads, kSmemBytes, stream_>>>(a);
-  else
-    k_gemm_tc<16><<<grid, kGemmThreads, kSmemBytes, stream_>>>(a);
-  O2F_CUDA(cudaGetLastError());
-  ++launches_;
+Mlp::~Mlp() {
+  // the destructor's frees wait for the device
+  if (graph_) cudaGraphExecDestroy(graph_);
+  for (auto& e : slot_free_)
+    if (e) cudaEventDestroy(e);
+  for (auto& e : fork_)
+    if (e) cudaEventDestroy(e);
+  if (join_) cudaEventDestroy(join_);
+  for (auto& c : capture_)
+    if (c) cudaStreamDestroy(c);
+  if (slots_) {
+    cudaStreamSynchronize(stream_);
+    cudaFreeHost(slots_);
+  }
 }
 
 GemmArgs Mlp::args() const {
@@ -199,65 +225,70 @@ GemmArgs Mlp::args() const {
   return a;
 }
 
-// Forward pass of n feature rows (X0_ filled): Z_/A_ per hidden layer, Y_.
-void Mlp::forward(int n) {
+// Forward pass of n feature rows (X0_ filled): Z_/A_ per hidden layer, the
+// first `outputs` columns of the last layer into y (row stride `outputs`).
+void Mlp::forward(int n, float* y, int outputs, cudaStream_t s) {
   const bf16* x = X0_;
   for (int l = 0; l <= kHidden; ++l) {
     GemmArgs a = args();
     a.M = n;
-    a.N = out_dim(l);
     a.K = in_dim(l);
     a.A = x;
-    a.sam = in_dim(l);
-    a.sak = 1;
+    a.lda = in_dim(l);
     a.B = Wb_[l];
-    a.sbn = in_dim(l);
-    a.sbk = 1;
-    a.k_split = a.K;
+    a.ldb = in_dim(l);
     a.bias = params_ + b_off_[l];
     if (l < kHidden) {
+      a.N = out_dim(l);
       a.epi = kEpiHidden;
       a.out = A_[l];
       a.pre = Z_[l];
       a.ldo = kWidth;
-      gemm(256, a, 1);
+      k_gemm_tc<64, false>
+          <<<dim3(blocks_of(n, kTileM), blocks_of(a.N, 64)), gemm_threads(64), gemm_smem_bytes<64>(), s>>>(a);
       x = A_[l];
     } else {
+      a.N = outputs;
       a.epi = kEpiLinear;
-      a.out32 = Y_;
-      a.ldo = kOutPad;
-      gemm(16, a, 1);
+      a.out32 = y;
+      a.ldo = outputs;
+      k_gemm_tc<16, false><<<dim3(blocks_of(n, kTileM), 1), gemm_threads(16), gemm_smem_bytes<16>(), s>>>(a);
     }
+    ++launches_;
   }
+  O2F_CUDA(cudaGetLastError());
 }
 
-// Backward pass from dY_ into grads_ (zeroed here).
-void Mlp::backward(int n) {
-  O2F_CUDA(cudaMemsetAsync(grads_, 0, n_params_ * sizeof(float), stream_));
+// Backward pass from dY_ into grads_ (zeroed here).  The chain of input
+// gradients runs on s; a layer's weight and bias gradients, which nothing in
+// the chain needs, on side (when it is another stream: a fork per layer and
+// one join).
+void Mlp::backward(int n, cudaStream_t s, cudaStream_t side) {
+  O2F_CUDA(cudaMemsetAsync(grads_, 0, n_params_ * sizeof(float), side));
   const bf16* g = dY_;  // gradient w.r.t. the output of layer l
-  bf16* bufs[2] = {dZa_, dZb_};
-  const int rows_split = 8;  // row slices of the bias column sums
   for (int l = kHidden; l >= 0; --l) {
     const int N = out_dim(l), K = in_dim(l);
-    const bf16* below = l > 0 ? A_[l - 1] : X0_;
-    // dW_l[n][k] = sum_m g(m, n) below(m, k): the batch is the reduction axis
+    if (side != s) {
+      O2F_CUDA(cudaEventRecord(fork_[l], s));
+      O2F_CUDA(cudaStreamWaitEvent(side, fork_[l], 0));
+    }
+    // dW_l[n][k] = sum_m g(m, n) below(m, k), db_l[n] = sum_m g(m, n): the
+    // batch is the reduction axis
     GemmArgs w = args();
     w.M = N;
     w.N = K;
     w.K = n;
     w.A = g;
-    w.sam = 1;
-    w.sak = N;
-    w.B = below;
-    w.sbn = 1;
-    w.sbk = K;
-    const int splits = std::max(1, std::min(64, (n + 2047) / 2048));
-    w.k_split = ((n + splits - 1) / splits + kKC - 1) / kKC * kKC;
+    w.lda = N;
+    w.B = l > 0 ? A_[l - 1] : X0_;
+    w.ldb = K;
     w.epi = kEpiAtomic;
     w.out32 = grads_ + w_off_[l];
+    w.bias_grad = grads_ + b_off_[l];
     w.ldo = K;
-    gemm(256, w, (n + w.k_split - 1) / w.k_split);
-    k_colsum<<<dim3(blocks_of(N, 128), rows_split), 128, 0, stream_>>>(n, N, g, grads_ + b_off_[l]);
+    k_gemm_tc<64, true><<<dim3(blocks_of(N, kTileM), blocks_of(K, 64), blocks_of(n, kMaxK)), gemm_threads(64),
+                          gemm_smem_bytes<64>(), side>>>(w);
+    ++launches_;
     if (l == 0) break;
     // gradient w.r.t. the layer below's pre-activation: (g W_l) * silu'(Z_{l-1})
     GemmArgs d = args();
@@ -265,26 +296,29 @@ void Mlp::backward(int n) {
     d.N = K;
     d.K = N;
     d.A = g;
-    d.sam = N;
-    d.sak = 1;
+    d.lda = N;
     d.B = WTb_[l];
-    d.sbn = N;
-    d.sbk = 1;
-    d.k_split = d.K;
+    d.ldb = N;
     d.epi = kEpiBackAct;
-    bf16* out = bufs[l & 1];
-    d.out = out;
+    d.out = dZ_[l - 1];  // one per layer: its weight gradient may still be reading it
     d.zprev = Z_[l - 1];
     d.ldo = kWidth;
-    gemm(256, d, 1);
-    g = out;
+    k_gemm_tc<64, false>
+        <<<dim3(blocks_of(n, kTileM), blocks_of(K, 64)), gemm_threads(64), gemm_smem_bytes<64>(), s>>>(d);
+    ++launches_;
+    g = dZ_[l - 1];
+  }
+  if (side != s) {
+    O2F_CUDA(cudaEventRecord(join_, side));
+    O2F_CUDA(cudaStreamWaitEvent(s, join_, 0));
   }
   O2F_CUDA(cudaGetLastError());
 }
 
-void Mlp::load_batch(const float* inputs_dev, const int* index_dev, int n) {
-  k_features<<<blocks_of(n, 128), 128, 0, stream_>>>(n, inputs_dev, index_dev, freq_, X0_);
+void Mlp::load_batch(const float* inputs_dev, const int* index_dev, int n, cudaStream_t s) {
+  k_features<<<blocks_of((int64_t)n * 32, 128), 128, 0, s>>>(n, inputs_dev, index_dev, freq_, X0_);
   O2F_CUDA(cudaGetLastError());
+  ++launches_;
 }
 
 void Mlp::set_data(const float* inputs, const float* targets, int64_t n) {
@@ -306,55 +340,107 @@ void Mlp::train(int steps, int batch, float lr, uint64_t seed, float* loss_hist)
   if (!(lr > 0.f)) throw Error(O2F_ERR_ARG, "lr must be positive");
   std::mt19937_64 rng(seed);
   std::uniform_int_distribution<int64_t> pick(0, n_data_ - 1);
-  std::vector<int> idx(batch);
   if (steps > loss_cap_) {
     loss_buf_ = arena_.alloc<float>(steps);
     loss_cap_ = steps;
   }
-  float* losses = loss_buf_;
-  O2F_CUDA(cudaMemsetAsync(losses, 0, steps * sizeof(float), stream_));
-  int* pinned = nullptr;
-  O2F_CUDA(cudaMallocHost(&pinned, sizeof(int) * batch));
+  O2F_CUDA(cudaMemsetAsync(loss_buf_, 0, steps * sizeof(float), stream_));
+  const size_t slot_ints = sizeof(StepHead) / sizeof(int) + (size_t)max_batch_;
+  if (!slots_) {
+    O2F_CUDA(cudaMallocHost(&slots_, kSlots * slot_ints * sizeof(int)));
+    for (auto& e : slot_free_) O2F_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto& e : fork_) O2F_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    O2F_CUDA(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
+    for (auto& c : capture_) O2F_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
+  }
+  build_graph(batch, lr);
+  // The host draws the batches some steps ahead of the device: pinned slots,
+  // each free again once its copy has been made.
+  for (int s = 0; s < steps; ++s) {
+    int* slot = slots_ + (size_t)(s % kSlots) * slot_ints;
+    if (s >= kSlots) O2F_CUDA(cudaEventSynchronize(slot_free_[s % kSlots]));
+    ++adam_t_;
+    const float b1 = 0.9f, b2 = 0.999f;
+    StepHead head{1.f - std::pow(b1, (float)adam_t_), 1.f - std::pow(b2, (float)adam_t_), s, 0};
+    std::memcpy(slot, &head, sizeof(head));
+    int* idx = slot + sizeof(StepHead) / sizeof(int);
+    for (int i = 0; i < batch; ++i) idx[i] = (int)pick(rng);
+    O2F_CUDA(cudaMemcpyAsync(step_in_, slot, sizeof(StepHead) + sizeof(int) * batch, cudaMemcpyHostToDevice, stream_));
+    O2F_CUDA(cudaEventRecord(slot_free_[s % kSlots], stream_));
+    O2F_CUDA(cudaGraphLaunch(graph_, stream_));
+    launches_ += graph_launches_;
+  }
+  sync();
+  if (loss_hist) O2F_CUDA(cudaMemcpy(loss_hist, loss_buf_, steps * sizeof(float), cudaMemcpyDeviceToHost));
+}
+
+// One training step as a graph: its batch, rates and loss place come from
+// step_in_.  Captured on streams of its own (the caller's may be one that
+// cannot be captured) and launched on the caller's.
+void Mlp::build_graph(int batch, float lr) {
+  if (graph_ && graph_batch_ == batch && graph_lr_ == lr && graph_data_ == data_in_ && graph_loss_ == loss_buf_) return;
+  if (graph_) {
+    O2F_CUDA(cudaGraphExecDestroy(graph_));
+    graph_ = nullptr;
+  }
+  cudaStream_t s = capture_[0], side = capture_[1];
+  const StepHead* head = reinterpret_cast<const StepHead*>(step_in_);
+  const int* index = step_in_ + sizeof(StepHead) / sizeof(int);
+  const int64_t before = launches_;
+  cudaGraph_t graph = nullptr;
+  O2F_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   try {
-    for (int s = 0; s < steps; ++s) {
-      for (int i = 0; i < batch; ++i) idx[i] = (int)pick(rng);
-      O2F_CUDA(cudaStreamSynchronize(stream_));  // the pinned index buffer is free again
-      std::memcpy(pinned, idx.data(), sizeof(int) * batch);
-      O2F_CUDA(cudaMemcpyAsync(index_, pinned, sizeof(int) * batch, cudaMemcpyHostToDevice, stream_));
-      load_batch(data_in_, index_, batch);
-      forward(batch);
-      k_loss<<<blocks_of(batch, 128), 128, 0, stream_>>>(batch, Y_, data_out_, index_, dY_, losses + s);
-      backward(batch);
-      ++adam_t_;
-      const float b1 = 0.9f, b2 = 0.999f;
-      const float c1 = 1.f - std::pow(b1, (float)adam_t_), c2 = 1.f - std::pow(b2, (float)adam_t_);
-      k_adam<<<blocks_of(n_params_, 256), 256, 0, stream_>>>(n_params_, params_, grads_, adam_m_, adam_v_, lr, b1,
-                                                             b2, 1e-8f, c1, c2);
-      pack();
-    }
-    sync();
+    load_batch(data_in_, index, batch, s);
+    forward(batch, Y_, kOutPad, s);
+    k_loss<<<blocks_of(batch, 128), 128, 0, s>>>(batch, Y_, data_out_, index, dY_, loss_buf_, head);
+    O2F_CUDA(cudaEventRecord(join_, s));
+    O2F_CUDA(cudaStreamWaitEvent(side, join_, 0));
+    backward(batch, s, side);
+    k_adam<<<blocks_of(n_params_, 256), 256, 0, s>>>(n_params_, params_, grads_, adam_m_, adam_v_, lr, 0.9f, 0.999f,
+                                                     1e-8f, head, layers());
+    O2F_CUDA(cudaGetLastError());
   } catch (...) {
-    cudaFreeHost(pinned);
+    cudaStreamEndCapture(s, &graph);
+    if (graph) cudaGraphDestroy(graph);
     throw;
   }
-  cudaFreeHost(pinned);
-  if (loss_hist) O2F_CUDA(cudaMemcpy(loss_hist, losses, steps * sizeof(float), cudaMemcpyDeviceToHost));
+  O2F_CUDA(cudaStreamEndCapture(s, &graph));
+  const cudaError_t e = cudaGraphInstantiate(&graph_, graph, 0);
+  cudaGraphDestroy(graph);
+  if (e != cudaSuccess) graph_ = nullptr;
+  O2F_CUDA(e);
+  graph_launches_ = launches_ - before + 2;
+  launches_ = before;
+  graph_batch_ = batch;
+  graph_lr_ = lr;
+  graph_data_ = data_in_;
+  graph_loss_ = loss_buf_;
+}
+
+Layers Mlp::layers() const {
+  Layers ly{};
+  for (int l = 0; l <= kHidden; ++l) {
+    ly.w_off[l] = w_off_[l];
+    ly.w_end[l] = b_off_[l];
+    ly.rows[l] = out_dim(l);
+    ly.cols[l] = in_dim(l);
+    ly.W[l] = Wb_[l];
+    ly.WT[l] = WTb_[l];
+  }
+  return ly;
 }
 
 void Mlp::predict(const float* inputs, int64_t n, float* out) {
   if (n <= 0) return;
   float* in_dev = arena_scratch_in(n);
   O2F_CUDA(cudaMemcpyAsync(in_dev, inputs, n * kIn * sizeof(float), cudaMemcpyHostToDevice, stream_));
-  std::vector<float> y((size_t)max_batch_ * kOutPad);
   for (int64_t b0 = 0; b0 < n; b0 += max_batch_) {
     const int m = (int)std::min<int64_t>(max_batch_, n - b0);
-    load_batch(in_dev + b0 * kIn, nullptr, m);
-    forward(m);
-    O2F_CUDA(cudaMemcpyAsync(y.data(), Y_, (size_t)m * kOutPad * sizeof(float), cudaMemcpyDeviceToHost, stream_));
-    sync();
-    for (int i = 0; i < m; ++i)
-      for (int j = 0; j < kOut; ++j) out[(b0 + i) * kOut + j] = y[(size_t)i * kOutPad + j];
+    load_batch(in_dev + b0 * kIn, nullptr, m, stream_);
+    forward(m, Y_, kOut, stream_);
+    O2F_CUDA(cudaMemcpyAsync(out + b0 * kOut, Y_, (size_t)m * kOut * sizeof(float), cudaMemcpyDeviceToHost, stream_));
   }
+  sync();
 }
 
 float* Mlp::arena_scratch_in(int64_t n) {
@@ -372,10 +458,10 @@ void Mlp::gradients(const float* inputs, const float* targets, int n, float* gra
   O2F_CUDA(cudaMemcpyAsync(in_dev, inputs, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice, stream_));
   O2F_CUDA(cudaMemcpyAsync(grad_targets_, targets, (size_t)n * kOut * sizeof(float), cudaMemcpyHostToDevice, stream_));
   O2F_CUDA(cudaMemsetAsync(loss_, 0, sizeof(float), stream_));
-  load_batch(in_dev, nullptr, n);
-  forward(n);
-  k_loss<<<blocks_of(n, 128), 128, 0, stream_>>>(n, Y_, grad_targets_, nullptr, dY_, loss_);
-  backward(n);
+  load_batch(in_dev, nullptr, n, stream_);
+  forward(n, Y_, kOutPad, stream_);
+  k_loss<<<blocks_of(n, 128), 128, 0, stream_>>>(n, Y_, grad_targets_, nullptr, dY_, loss_, nullptr);
+  backward(n, stream_, stream_);
   sync();
   O2F_CUDA(cudaMemcpy(grads_out, grads_, n_params_ * sizeof(float), cudaMemcpyDeviceToHost));
   if (loss_out) O2F_CUDA(cudaMemcpy(loss_out, loss_, sizeof(float), cudaMemcpyDeviceToHost));

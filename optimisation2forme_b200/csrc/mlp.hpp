@@ -11,10 +11,14 @@ namespace o2f {
 namespace mlp {
 
 struct GemmArgs;
+struct Layers;
 
 class Mlp {
  public:
   Mlp(int max_batch, float freq_scale, uint64_t seed, cudaStream_t stream);
+  ~Mlp();
+  Mlp(const Mlp&) = delete;
+  Mlp& operator=(const Mlp&) = delete;
   int64_t n_params() const { return n_params_; }
   void set_data(const float* inputs, const float* targets, int64_t n);
   void train(int steps, int batch, float lr, uint64_t seed, float* loss_hist);
@@ -27,11 +31,12 @@ class Mlp {
  private:
   void sync();
   void pack();
-  void gemm(int nt, const GemmArgs& a, int splits);
   GemmArgs args() const;
-  void forward(int n);
-  void backward(int n);
-  void load_batch(const float* inputs_dev, const int* index_dev, int n);
+  Layers layers() const;
+  void forward(int n, float* y, int outputs, cudaStream_t s);
+  void backward(int n, cudaStream_t s, cudaStream_t side);
+  void load_batch(const float* inputs_dev, const int* index_dev, int n, cudaStream_t s);
+  void build_graph(int batch, float lr);
   float* arena_scratch_in(int64_t n);
 
   int max_batch_;
@@ -44,8 +49,8 @@ class Mlp {
   __nv_bfloat16* X0_ = nullptr;
   __nv_bfloat16 *Z_[4]{}, *A_[4]{};
   float* Y_ = nullptr;
-  __nv_bfloat16 *dY_ = nullptr, *dZa_ = nullptr, *dZb_ = nullptr;
-  int* index_ = nullptr;
+  __nv_bfloat16 *dY_ = nullptr, *dZ_[4]{};
+  int* step_in_ = nullptr;  // head and row indices of a training step
   float* loss_ = nullptr;
   int* err_ = nullptr;
   float *data_in_ = nullptr, *data_out_ = nullptr;
@@ -57,6 +62,16 @@ class Mlp {
   float* grad_targets_ = nullptr;
   int64_t adam_t_ = 0;
   int64_t launches_ = 0;
+  // training: pinned copies of step_in_ that the host fills ahead, the step's graph
+  static constexpr int kSlots = 4;
+  int* slots_ = nullptr;
+  cudaEvent_t slot_free_[kSlots]{}, fork_[5]{}, join_ = nullptr;
+  cudaStream_t capture_[2]{};
+  cudaGraphExec_t graph_ = nullptr;
+  int64_t graph_launches_ = 0;
+  int graph_batch_ = 0;
+  float graph_lr_ = 0.f;
+  const float *graph_data_ = nullptr, *graph_loss_ = nullptr;
 };
 
 }  // namespace mlp
