@@ -708,6 +708,19 @@ __global__ void k_vertex_weights(int64_t n, const int32_t* __restrict__ verts, c
   }
 }
 
+// A per-cell vector from and to the reference's cell order (ref[c]: reference
+// number of cell c).
+__global__ void k_from_reference_order(int64_t nc, const int32_t* __restrict__ ref, const Vec4<double>* __restrict__ x,
+                                       Vec4<double>* __restrict__ y) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < nc) y[c] = x[ref[c]];
+}
+__global__ void k_to_reference_order(int64_t nc, const int32_t* __restrict__ ref, const Vec4<double>* __restrict__ x,
+                                     Vec4<double>* __restrict__ y) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < nc) y[ref[c]] = x[c];
+}
+
 // Uniform state fill (init_one_x, src/init.cpp:57-81), on the device.
 template <typename T>
 __global__ void k_fill_state(int64_t nc, Vec4<T> v, Vec4<T>* __restrict__ U) {

@@ -328,6 +328,11 @@ void Solver::upload_mesh() {
   h2d(topo_.pert_cells, pcells, s);
   h2d(topo_.pert_wverts, pwverts, s);
 
+  const std::vector<int32_t> ref_cell(cperm_.begin(), cperm_.end());
+  ref_cell_ = arena_.alloc<int32_t>(nc);
+  xfer_ = arena_.alloc<Vec4<double>>(nc);
+  h2d(ref_cell_, ref_cell, s);
+
   upload_geometry();
 
   work_ = alloc_work();
@@ -484,13 +489,9 @@ void Solver::render_field(const std::string& field, int nx, int ny, const std::s
     launch_residual(geom_, work_, U_, nullptr, true, nullptr);
     have_residual_ = true;
   }
-  if (!render_ref_id_) {
-    std::vector<int32_t> ids(nc);
-    for (int64_t c = 0; c < nc; ++c) ids[c] = (int32_t)cperm_[c];
-    render_ref_id_ = arena_.alloc<int32_t>(nc);
+  if (!render_scalar_) {
     render_scalar_ = arena_.alloc<double>(nc);
     render_part_ = arena_.alloc<double>(2 * 1184);
-    h2d(render_ref_id_, ids, s);
   }
   k_cell_scalar<<<grid(nc), kBlock, 0, s>>>(nc, U_, work_.grad, f, params_.gamma, render_scalar_);
   const int parts = std::min(grid(nc), 1184);
@@ -542,7 +543,7 @@ void Solver::render_field(const std::string& field, int nx, int ny, const std::s
   auto* img = static_cast<unsigned char*>(img_buf.p);
   RenderView w{x_min, y_min, std::abs(x_max - x_min), std::abs(y_max - y_min), nx, ny};
   O2F_CUDA(cudaMemsetAsync(pix, 0xff, npix * sizeof(unsigned long long), s));
-  k_raster_cells<<<grid(nc), kBlock, 0, s>>>(nc, topo_.cverts, topo_.ctype, geom_.vxy, render_ref_id_, w, pix);
+  k_raster_cells<<<grid(nc), kBlock, 0, s>>>(nc, topo_.cverts, topo_.ctype, geom_.vxy, ref_cell_, w, pix);
   k_colour_pixels<<<(int)((npix + kBlock - 1) / kBlock), kBlock, 0, s>>>(nx, ny, pix, render_scalar_, fmin_, span,
                                                                          cmap == "schlieren" ? 1 : 0, img);
   O2F_CUDA(cudaGetLastError());
@@ -846,29 +847,24 @@ o2f_mesh_info Solver::info() const {
 
 int64_t Solver::export_array(const std::string& w, void* out) const { return export_mesh_array(hm_, w, out); }
 
+// Per-cell vectors cross the boundary in the reference's cell order and are
+// reordered on the device: the host's part is the copy alone (with the
+// reordering on the host, through a temporary, 2.0M cells took 21-35 ms each
+// way).
 void Solver::to_internal(const double* ref, Vec4<double>* dev) {
-  const int64_t nc = hm_.nc;
-  std::vector<Vec4<double>> tmp(nc);
-  for (int64_t c = 0; c < nc; ++c) {
-    const double* q = ref + 4 * cperm_[c];
-    tmp[c] = Vec4<double>{q[0], q[1], q[2], q[3]};
-  }
-  O2F_CUDA(cudaMemcpyAsync(dev, tmp.data(), nc * sizeof(Vec4<double>), cudaMemcpyHostToDevice, stream_));
+  const int64_t nc = topo_.nc;
+  O2F_CUDA(cudaMemcpyAsync(xfer_, ref, nc * sizeof(Vec4<double>), cudaMemcpyHostToDevice, stream_));
+  k_from_reference_order<<<grid(nc), kBlock, 0, stream_>>>(nc, ref_cell_, xfer_, dev);
+  O2F_CUDA(cudaGetLastError());
   sync();
 }
 
 void Solver::to_reference(const Vec4<double>* dev, double* ref) {
-  const int64_t nc = hm_.nc;
-  std::vector<Vec4<double>> tmp(nc);
-  O2F_CUDA(cudaMemcpyAsync(tmp.data(), dev, nc * sizeof(Vec4<double>), cudaMemcpyDeviceToHost, stream_));
+  const int64_t nc = topo_.nc;
+  k_to_reference_order<<<grid(nc), kBlock, 0, stream_>>>(nc, ref_cell_, dev, xfer_);
+  O2F_CUDA(cudaGetLastError());
+  O2F_CUDA(cudaMemcpyAsync(ref, xfer_, nc * sizeof(Vec4<double>), cudaMemcpyDeviceToHost, stream_));
   sync();
-  for (int64_t c = 0; c < nc; ++c) {
-    double* q = ref + 4 * cperm_[c];
-    q[0] = tmp[c].a;
-    q[1] = tmp[c].b;
-    q[2] = tmp[c].c;
-    q[3] = tmp[c].d;
-  }
 }
 
 void Solver::state_set(const double* U_ref) {

@@ -178,6 +178,8 @@ class Solver {
   Topo topo_{};
   Geom<double> geom_{};
   Work<double> work_{};
+  int32_t* ref_cell_ = nullptr;     // [nc] reference number of each cell
+  Vec4<double>* xfer_ = nullptr;    // [nc] a vector in reference order, on its way to or from the host
   Vec4<double>* U_ = nullptr;
   Vec4<double>* Uold_ = nullptr;
   bool f32_ready_ = false;
@@ -245,7 +247,6 @@ class Solver {
   int32_t* idw_src_ = nullptr;
   Vec2<double>*idw_sxy_ = nullptr, *idw_sd_ = nullptr, *dvxy_ = nullptr;
   // field images
-  int32_t* render_ref_id_ = nullptr;
   double *render_scalar_ = nullptr, *render_part_ = nullptr;
   double last_residual_ms_ = 0.0;
   int64_t launches_ = 0;
