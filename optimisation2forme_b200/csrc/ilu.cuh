@@ -27,67 +27,6 @@
 
 namespace o2f {
 
-__device__ __forceinline__ void mat4_mul(const double* a, const double* b, double* c) {
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      c[r * 4 + q] = a[r * 4 + 0] * b[0 * 4 + q] + a[r * 4 + 1] * b[1 * 4 + q] + a[r * 4 + 2] * b[2 * 4 + q] +
-                     a[r * 4 + 3] * b[3 * 4 + q];
-}
-
-// 4x4 inverse by Gauss-Jordan elimination with partial pivoting; returns
-// false for a singular block (the inverse is then set to the identity).
-__device__ __forceinline__ bool mat4_inv(const double* a_in, double* inv) {
-  double a[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    a[i] = a_in[i];
-    inv[i] = (i % 5 == 0) ? 1.0 : 0.0;
-  }
-  for (int col = 0; col < 4; ++col) {
-    int piv = col;
-    double best = fabs(a[col * 4 + col]);
-    for (int r = col + 1; r < 4; ++r) {
-      const double v = fabs(a[r * 4 + col]);
-      if (v > best) {
-        best = v;
-        piv = r;
-      }
-    }
-    if (!(best > 0.0)) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) inv[i] = (i % 5 == 0) ? 1.0 : 0.0;
-      return false;
-    }
-    if (piv != col) {
-      for (int q = 0; q < 4; ++q) {
-        double t = a[col * 4 + q];
-        a[col * 4 + q] = a[piv * 4 + q];
-        a[piv * 4 + q] = t;
-        t = inv[col * 4 + q];
-        inv[col * 4 + q] = inv[piv * 4 + q];
-        inv[piv * 4 + q] = t;
-      }
-    }
-    const double d = 1.0 / a[col * 4 + col];
-    for (int q = 0; q < 4; ++q) {
-      a[col * 4 + q] *= d;
-      inv[col * 4 + q] *= d;
-    }
-    for (int r = 0; r < 4; ++r) {
-      if (r == col) continue;
-      const double f = a[r * 4 + col];
-      if (f == 0.0) continue;
-      for (int q = 0; q < 4; ++q) {
-        a[r * 4 + q] -= f * a[col * 4 + q];
-        inv[r * 4 + q] -= f * inv[col * 4 + q];
-      }
-    }
-  }
-  return true;
-}
-
 // Assemble the block rows of A from the Jacobian blocks of k_jt_blocks.
 __global__ void __launch_bounds__(kBlock) k_ilu_assemble(int64_t nc, const int32_t* __restrict__ jslot, Geom<double> g,
                                                          const int2* __restrict__ ec,
@@ -137,56 +76,150 @@ __global__ void __launch_bounds__(kBlock) k_ilu_assemble(int64_t nc, const int32
   for (int i = 0; i < 16; ++i) row[i] = diag[i];
 }
 
-// One level of the factorization.
-__global__ void __launch_bounds__(128) k_ilu_factor(const int32_t* __restrict__ cells, int n, IluDev ilu,
-                                                    int* status) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int i = cells[t];
-  const int64_t nc = ilu.nc;
-  double* row = ilu.A + (int64_t)i * 80;
-  const int pi = ilu.pos[i];
-  int nb[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) nb[k] = ilu.nbr[(int64_t)k * nc + i];
-  // lower neighbours in increasing ILU position
-  int order[4], nlow = 0;
-  for (int k = 0; k < 4; ++k)
-    if (nb[k] >= 0 && ilu.pos[nb[k]] < pi) order[nlow++] = k;
-  for (int a = 1; a < nlow; ++a)
-    for (int b = a; b > 0 && ilu.pos[nb[order[b]]] < ilu.pos[nb[order[b - 1]]]; --b) {
-      const int tmp = order[b];
-      order[b] = order[b - 1];
-      order[b - 1] = tmp;
-    }
-  double L[16], prod[16];
-  for (int a = 0; a < nlow; ++a) {
-    const int slot = order[a];
-    const int k = nb[slot];
-    double* Aik = row + 16 * (1 + slot);
-    mat4_mul(Aik, ilu.Dinv + (int64_t)k * 16, L);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) Aik[q] = L[q];
-    // subtract L_ik U_kj for the upper blocks j of row k held by row i
-    const double* rowk = ilu.A + (int64_t)k * 80;
-    const int pk = ilu.pos[k];
-    for (int m = 0; m < 4; ++m) {
-      const int j = ilu.nbr[(int64_t)m * nc + k];
-      if (j < 0 || ilu.pos[j] <= pk) continue;
-      double* dst = nullptr;
-      if (j == i) {
-        dst = row;
-      } else {
-        for (int s = 0; s < 4; ++s)
-          if (nb[s] == j) dst = row + 16 * (1 + s);
+// One level of the factorization.  Sixteen lanes solve a row, one matrix
+// element each: a level is bound by the latency of its rows, and with a
+// thread per row that was a chain of some 700 FP64 operations through local
+// memory.  What a solve costs besides its iterations, most of it here: 75k
+// rows 16 -> 4.1 ms, and 2.8 with the levels overlapped as below; 300k rows
+// 36 -> 9.1 -> 5.8.  Every element sees the operations of Gauss-Jordan
+// elimination with partial pivoting, and of the block products, in the same
+// order.
+constexpr int kFactorBlock = 128;
+constexpr int kFactorRows = kFactorBlock / 16;
+
+__device__ __forceinline__ double lane16(double v, int src) { return __shfl_sync(0xffffffffu, v, src, 16); }
+__device__ __forceinline__ int lane16(int v, int src) { return __shfl_sync(0xffffffffu, v, src, 16); }
+
+// Element (r, q) of the inverse of the block whose element (r, q) is a; false
+// for a singular block (the inverse is then the identity).
+__device__ __forceinline__ bool mat4_inv16(double a, int r, int q, double& inv) {
+  const double one = r == q ? 1.0 : 0.0;
+  inv = one;
+  bool regular = true;
+  for (int col = 0; col < 4; ++col) {
+    int piv = col;
+    double best = fabs(lane16(a, col * 5));
+    for (int k = col + 1; k < 4; ++k) {
+      const double v = fabs(lane16(a, k * 4 + col));
+      if (v > best) {
+        best = v;
+        piv = k;
       }
-      if (!dst) continue;
-      mat4_mul(L, rowk + 16 * (1 + m), prod);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) dst[q] -= prod[q];
+    }
+    if (!(best > 0.0)) regular = false;
+    // rows col and piv change places
+    const int from = (r == col ? piv : r == piv ? col : r) * 4 + q;
+    a = lane16(a, from);
+    inv = lane16(inv, from);
+    const double d = 1.0 / lane16(a, col * 5);
+    if (r == col) {
+      a *= d;
+      inv *= d;
+    }
+    const double f = lane16(a, r * 4 + col), pa = lane16(a, col * 4 + q), pi = lane16(inv, col * 4 + q);
+    if (r != col && f != 0.0) {
+      a -= f * pa;
+      inv -= f * pi;
     }
   }
-  if (!mat4_inv(row, ilu.Dinv + (int64_t)i * 16)) atomicExch(status, 1);
+  if (!regular) inv = one;
+  return regular;
+}
+
+// A level may start while the one before it runs (all launches but the
+// first): it then loads its own rows, which no other level writes, and waits
+// for that level's results.  It lets its successor start after that wait, so
+// that the assembled rows are complete when any level reads them.
+__global__ void __launch_bounds__(kFactorBlock) k_ilu_factor(const int32_t* __restrict__ cells, int n, IluDev ilu,
+                                                             int* status) {
+  const int t = (blockIdx.x * kFactorBlock + threadIdx.x) >> 4;
+  const int e = threadIdx.x & 15, r = e >> 2, q = e & 3;
+  const bool mine = t < n;
+  const int64_t nc = ilu.nc;
+  const int i = mine ? cells[t] : 0;
+  double* row = ilu.A + (int64_t)i * 80;
+  const int pi = mine ? ilu.pos[i] : 0;
+  // lane 4 k + m: neighbour m of neighbour k
+  const int nk = mine ? ilu.nbr[(int64_t)r * nc + i] : -1;
+  const int pk_e = nk >= 0 ? ilu.pos[nk] : -1;
+  const int j_e = nk >= 0 ? ilu.nbr[(int64_t)q * nc + nk] : -1;
+  const int pj_e = j_e >= 0 ? ilu.pos[j_e] : -1;
+  double blk[5];
+#pragma unroll
+  for (int b = 0; b < 5; ++b) blk[b] = mine ? row[16 * b + e] : 0.0;
+  int nb[4], pk[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    nb[k] = lane16(nk, 4 * k);
+    pk[k] = lane16(pk_e, 4 * k);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (nk >= 0 && pk_e < pi) {  // one line a block: the factors this row will read
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(ilu.A + (int64_t)nk * 80 + 16 * (1 + q)));
+    if (q == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(ilu.Dinv + (int64_t)nk * 16));
+  }
+  // lower neighbours in increasing ILU position (equal ones in slot order)
+  int last = -1, last_slot = -1;
+  for (int a = 0; a < 4; ++a) {
+    int slot = -1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool low = nb[k] >= 0 && pk[k] < pi && (pk[k] > last || (pk[k] == last && k > last_slot));
+      if (low && (slot < 0 || pk[k] < pk[slot < 0 ? 0 : slot])) slot = k;
+    }
+    const bool on = slot >= 0;
+    if (!__any_sync(0xffffffffu, on)) break;
+    int kc = 0, pks = 0;
+    double aik = 0.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (slot == k) {
+        kc = nb[k];
+        pks = pk[k];
+        aik = blk[1 + k];
+      }
+    if (on) {
+      last = pks;
+      last_slot = slot;
+    }
+    // L = A_ik D_k^{-1}
+    const double* D = ilu.Dinv + (int64_t)(on ? kc : i) * 16 + q;
+    const double L = lane16(aik, 4 * r) * (on ? D[0] : 0.0) + lane16(aik, 4 * r + 1) * (on ? D[4] : 0.0) +
+                     lane16(aik, 4 * r + 2) * (on ? D[8] : 0.0) + lane16(aik, 4 * r + 3) * (on ? D[12] : 0.0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (slot == k) blk[1 + k] = L;
+    const double l0 = lane16(L, 4 * r), l1 = lane16(L, 4 * r + 1), l2 = lane16(L, 4 * r + 2), l3 = lane16(L, 4 * r + 3);
+    // subtract L_ik U_kj for the upper blocks j of row k held by row i
+    const double* rowk = ilu.A + (int64_t)(on ? kc : i) * 80;
+    for (int m = 0; m < 4; ++m) {
+      const int j = lane16(j_e, 4 * (on ? slot : 0) + m), pj = lane16(pj_e, 4 * (on ? slot : 0) + m);
+      int dst = -1;
+      if (on && j >= 0 && pj > pks) {
+        if (j == i) {
+          dst = 0;
+        } else {
+#pragma unroll
+          for (int s = 0; s < 4; ++s)
+            if (nb[s] == j) dst = 1 + s;
+        }
+      }
+      if (dst < 0) continue;
+      const double* U = rowk + 16 * (1 + m) + q;
+      const double prod = l0 * U[0] + l1 * U[4] + l2 * U[8] + l3 * U[12];
+#pragma unroll
+      for (int b = 0; b < 5; ++b)
+        if (dst == b) blk[b] -= prod;
+    }
+  }
+  double inv;
+  const bool regular = mat4_inv16(blk[0], r, q, inv);
+  if (!mine) return;
+#pragma unroll
+  for (int b = 0; b < 5; ++b) row[16 * b + e] = blk[b];
+  ilu.Dinv[(int64_t)i * 16 + e] = inv;
+  if (!regular && e == 0) atomicExch(status, 1);
 }
 
 // Sync-free triangular sweeps (one launch per triangle).  Rows are processed

@@ -672,7 +672,6 @@ void Solver::setup_ilu_host(const std::vector<int32_t>& jslot, const std::vector
     for (int64_t i = nc - 1; i >= 0; --i) ilu_sweep_h_[nc + fill[levu[order[i]]]++] = order[i];
   }
   ilu_n_up_ = nup;
-  ilu_plan_h_ = make_sweep_plan(nc, ilu_nbr_h_, ilu_pos_h_, order);
   ilu_order_h_ = std::move(order);
   ilu_.nc = nc;
   ilu_.n_lo = nlo;
@@ -692,6 +691,8 @@ void Solver::ilu_factor() {
     ilu_.Dinv = arena_.alloc<double>(16 * nc);
     ilu_.order = arena_.alloc<int32_t>(nc);
     ilu_.sweep = arena_.alloc<int32_t>(2 * nc);
+    // made here: a context that only steps in time has no use for it
+    ilu_plan_h_ = make_sweep_plan(nc, ilu_nbr_h_, ilu_pos_h_, ilu_order_h_);
     const SweepPlan& pl = ilu_plan_h_;
     if (pl.cluster > 0) {
       ilu_.cl_blocks = pl.cluster;
@@ -736,7 +737,17 @@ void Solver::ilu_factor() {
                                                params_.adjoint_shift, ilu_);
   for (int l = 0; l < ilu_.n_lo; ++l) {
     const int n = lo_off_h_[l + 1] - lo_off_h_[l];
-    k_ilu_factor<<<(n + 127) / 128, 128, 0, s>>>(ilu_.lo_cells + lo_off_h_[l], n, ilu_, ilu_status_);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((n + kFactorRows - 1) / kFactorRows);
+    cfg.blockDim = dim3(kFactorBlock);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = l > 0 ? 1 : 0;
+    O2F_CUDA(cudaLaunchKernelEx(&cfg, k_ilu_factor, static_cast<const int32_t*>(ilu_.lo_cells + lo_off_h_[l]), n, ilu_,
+                                ilu_status_));
   }
   // the factor blocks in the block sweeps' order
   if (ilu_block_sweeps()) {
