@@ -423,22 +423,31 @@ __global__ void __launch_bounds__(kSweepBlock) k_ilu_sweep(int n, IluDev ilu, co
 //     levels, arrived at that long before it is waited for, which bounds how
 //     far blocks run apart and so makes slots and barriers reusable);
 //   * factor blocks, D^-1 (backward), own values and records of the next
-//     kStageRing levels are copied into shared memory by a warp of its own
-//     (bulk copies, contiguous in sweep order), and are in a row's registers
-//     before the level begins.
+//     kStageRing levels are copied into shared memory by warps of their own,
+//     one per slot of the ring (bulk copies, contiguous in sweep order; to
+//     start a level's takes a thread 1,000 cycles), and are in a row's
+//     registers, with the addresses it stores to, before the level begins:
+//     two sets of warps take turns, so that a set has two levels for that.
 // Four lanes solve a row (one component each), eight warps the kSweepChunks
 // chunks of a block.  The arithmetic of a row (dependencies in slot order)
 // is that of k_ilu_sweep: both give the same bits.
-// Measured on B200, ms per adjoint iteration (four sweeps) alone: 1.08 at
-// 74,528 rows, 2.29 at 300,300, against 3.93 and 13.1 for one block walking
-// plain levels behind a block barrier and 5.2 and 11.6 for k_ilu_sweep; about
-// 1,000 cycles a level, of them 270 (forward) to 390 (backward) the dot and
-// some 600 from store to reader.  Slower, and not kept: a cluster barrier
-// with release per level (3.0 ms at 74,528 rows: the release waits for the
-// level's global stores, 1,400 cycles), operand slots that are polled for a
-// sentinel instead of barriers that are waited on (1.27 ms), 16-byte instead
-// of 8-byte stores per lane (1.18 against 1.13 ms).
-constexpr int kSweepThreads = 128 * kSweepChunks + 32 * (kSweepChunks + 2);
+// Measured on B200, ms per adjoint iteration (four sweeps) alone: 0.96 at
+// 74,528 rows, 1.96 at 300,300, against 3.93 and 13.1 for one block walking
+// plain levels behind a block barrier and 5.2 and 11.6 for k_ilu_sweep, 1.09
+// and 2.31 with one set of warps and one staging warp per chunk.  About 900
+// cycles a level, of them 550 (forward) to 800 (backward) from the barrier to
+// the stores; a warp's two levels are filled by 135 cycles of the cluster
+// barrier, 250 of waiting, 650 of loading the next row.  Slower, and not kept: a
+// cluster barrier with release per level (3.0 ms at 74,528 rows: the release
+// waits for the level's global stores, 1,400 cycles), operand slots that are
+// polled for a sentinel instead of barriers that are waited on (1.27 ms),
+// 16-byte instead of 8-byte stores per lane (1.18 against 1.13 ms), plain
+// shared stores and an arrival per warp for values that stay in the block
+// (1.01 against 0.96 ms), four copies started by one instruction (1.45
+// against 1.17 ms).
+constexpr int kSweepWarps = 4 * kSweepChunks;  // of a level
+constexpr int kStageRing = 4;  // levels staged at once
+constexpr int kSweepThreads = 32 * (2 * kSweepWarps + kStageRing + 2);
 constexpr int kSweepWindow = 2048;  // operand slots (32 B each)
 static_assert(kSweepWindow == kSweepSlots && (kSweepSlots & (kSweepSlots - 1)) == 0, "operand slots");
 constexpr int kStageSlots = 3;      // dependencies whose blocks are staged (the third where a row of the chunk has one)
@@ -448,7 +457,6 @@ constexpr int kStageChunksBwd = 2;
 static_assert(kStageChunksFwd == kSweepChunks && kStageChunksBwd == kSweepChunks, "every chunk of a block is staged");
 constexpr int kStageBwdD = kStageChunksBwd * kStageChunkDoubles;  // offset of the staged D^-1, doubles
 constexpr int kStageDoubles = kStageBwdD + kStageChunksBwd * 512;  // blocks (and D^-1) of one level
-constexpr int kStageRing = 4;       // levels staged at once
 constexpr int kStageOwn = kSweepChunks * 128;  // own values of one level, doubles
 constexpr int kRecChunkBytes = 32 * kSweepRec * 4;
 constexpr int kL2Lead = 16;         // levels between the L2 prefetch of a level's blocks and its use
@@ -575,8 +583,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
   if (threadIdx.x == 0) {
     for (int i = 0; i < kSweepBars; ++i) bar_init(bar_op + 8u * i, 1);
     for (int i = 0; i < kStageRing; ++i) {
-      bar_init(bar_full + 8u * i, kSweepChunks);
-      bar_init(bar_empty + 8u * i, 4 * kSweepChunks);
+      bar_init(bar_full + 8u * i, 1);
+      bar_init(bar_empty + 8u * i, kSweepWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -593,82 +601,103 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
     cluster_arrive();
   };
 
-  // Helper warps, one thread of each at work: one per chunk that stages its
-  // copies, one that sets what each level's barrier waits for, one that
-  // requests blocks into L2 (a single thread for all took longer than a level).
-  if (warp >= 4 * kSweepChunks) {
+  // Helper warps: one per staging slot, whose first thread starts the slot's
+  // copies (they take it longer than a level), one that sets what each level's
+  // barrier waits for, one that requests blocks into L2.
+  if (warp >= 2 * kSweepWarps) {
     const int32_t* __restrict__ rec = ilu.cl_rec[kDir];
     const double* __restrict__ pack = ilu.pack[kDir];
     const double* own = reinterpret_cast<const double*>(kForward ? ilu.own_f : ilu.own_b);
-    const int j = warp - 4 * kSweepChunks;
-    // A level's barrier is set kSweepNear levels ahead: by then every warp
-    // has left the level that used it last (kSweepSkew levels back), so a
-    // phase that has nothing to wait for cannot pass one that is waited on.
-    const int kLead = j < kSweepChunks ? kStageRing : j == kSweepChunks ? kSweepNear : kL2Lead;
+    const int slot = warp - 2 * kSweepWarps;
     auto info_of = [&](int l) { return l < nlev ? info[(int64_t)l * C] : make_int4(0, -1, 0, 0); };
-    auto work = [&](int l, const int4& in) {
-      if (in.y < 0) return;
-      if (j < kSweepChunks) {
-        const int slot = l % kStageRing;
-        const uint32_t bar = bar_full + 8u * slot;
-        if (j == 0) s_cnt[slot] = in.y;
-        if (j >= in.y) {
-          bar_arrive(bar);
-          return;
-        }
-        const uint32_t blk = (in.z >> j & 1 ? 3 : 2) * 4096;
-        const int64_t k = in.x + (int64_t)j * C;
+    if (slot < kStageRing) {
+      const uint32_t bar = bar_full + 8u * slot;
+      auto stage = [&](const int4& in) {
+        if (in.y < 0) return;
+        s_cnt[slot] = in.y;
+        uint32_t bytes = 0;
+        for (int j = 0; j < in.y; ++j)
+          bytes += 1024 + kRecChunkBytes + (kForward ? 0 : 4096) + (in.z >> j & 1 ? 3 : 2) * 4096;
+        bar_expect(bar, bytes);
         const uint32_t dst = sweep_smem(s_blk + slot * kStageDoubles);
-        bar_expect(bar, 1024 + kRecChunkBytes + (kForward ? 0 : 4096) + blk);
-        bulk_copy(dst + (uint32_t)j * kStageChunkDoubles * 8, pack + k * 2048, blk, bar);
-        if (!kForward) bulk_copy(dst + (uint32_t)(kStageBwdD + j * 512) * 8, ilu.packD + k * 512, 4096, bar);
-        bulk_copy(sweep_smem(s_rec) + (uint32_t)(slot * kSweepChunks + j) * kRecChunkBytes,
-                  rec + k * 32 * kSweepRec, kRecChunkBytes, bar);
-        bulk_copy(sweep_smem(s_own + slot * kStageOwn + j * 128), own + k * 128, 1024, bar);
-      } else if (j == kSweepChunks) {
-        bar_expect(bar_op + 8u * (l % kSweepBars), (uint32_t)in.w);
-      } else {
-        for (int i = 0; i < in.y; ++i) {
-          const int64_t k = in.x + (int64_t)i * C;
-          prefetch_l2_bulk(pack + k * 2048, 8192);
-          if (!kForward) prefetch_l2_bulk(ilu.packD + k * 512, 4096);
+        for (int j = 0; j < in.y; ++j) {
+          const int64_t k = in.x + (int64_t)j * C;
+          bulk_copy(dst + (uint32_t)j * kStageChunkDoubles * 8, pack + k * 2048, (in.z >> j & 1 ? 3 : 2) * 4096, bar);
+          if (!kForward) bulk_copy(dst + (uint32_t)(kStageBwdD + j * 512) * 8, ilu.packD + k * 512, 4096, bar);
+          bulk_copy(sweep_smem(s_rec) + (uint32_t)(slot * kSweepChunks + j) * kRecChunkBytes,
+                    rec + k * 32 * kSweepRec, kRecChunkBytes, bar);
+          bulk_copy(sweep_smem(s_own + slot * kStageOwn + j * 128), own + k * 128, 1024, bar);
+        }
+      };
+      int4 next{};
+      if (lane == 0) {
+        stage(info_of(slot));
+        next = info_of(slot + kStageRing);
+      }
+      for (int l = slot; l - slot < nlev; l += kStageRing) {
+        keep_together(l - slot);
+        if (lane == 0 && l < nlev) {
+          const int4 in = next;
+          next = info_of(l + 2 * kStageRing);
+          bar_wait(bar_empty + 8u * slot, (l / kStageRing) & 1, bad);
+          if (!bad) stage(in);
         }
       }
-    };
-    int4 next{};
-    if (lane == 0) {
-      for (int l = 0; l < kLead; ++l) work(l, info_of(l));
-      next = info_of(kLead);
-    }
-    for (int l = 0; l < nlev; ++l) {
-      keep_together(l);
-      if (lane == 0) {
-        const int4 in = next;
-        next = info_of(l + 1 + kLead);
-        if (j < kSweepChunks)
-          bar_wait(bar_empty + 8u * (l % kStageRing), (l / kStageRing) & 1, bad);
-        else if (j > kSweepChunks)
-          bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
+    } else {
+      // A level's barrier is set kSweepNear levels ahead: by then every warp
+      // has left the level that used it last (kSweepSkew levels back), so a
+      // phase that has nothing to wait for cannot pass one that is waited on.
+      const bool arms = slot == kStageRing;
+      const int kLead = arms ? kSweepNear : kL2Lead;
+      auto work = [&](int l, const int4& in) {
+        if (in.y < 0) return;
+        if (arms) {
+          if (lane == 0) bar_expect(bar_op + 8u * (l % kSweepBars), (uint32_t)in.w);
+        } else if (lane < 2 * kSweepChunks && (lane >> 1) < in.y && !(kForward && (lane & 1))) {
+          const int64_t k = in.x + (int64_t)(lane >> 1) * C;
+          prefetch_l2_bulk(lane & 1 ? ilu.packD + k * 512 : pack + k * 2048, lane & 1 ? 4096 : 8192);
+        }
+      };
+      // entries of 32 levels, one a lane, and the 32 after them
+      int4 now = info_of(lane), then = info_of(32 + lane);
+      auto entry = [&](int l) {
+        if (l && l % 32 == 0) {
+          now = then;
+          then = info_of(l + 32 + lane);
+        }
+        return make_int4(__shfl_sync(0xffffffffu, now.x, l % 32), __shfl_sync(0xffffffffu, now.y, l % 32),
+                         __shfl_sync(0xffffffffu, now.z, l % 32), __shfl_sync(0xffffffffu, now.w, l % 32));
+      };
+      for (int l = 0; l < kLead; ++l) work(l, entry(l));
+      for (int l = 0; l < nlev; ++l) {
+        keep_together(l);
+        const int4 in = entry(l + kLead);
+        if (!arms) bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
+        bad = __any_sync(0xffffffffu, bad);
         if (!bad) work(l + kLead, in);
       }
     }
   } else {
-    const int j = warp >> 2, q = (warp & 3) * 8 + (lane >> 2), c = lane & 3;
+    const int set = warp / kSweepWarps, j = (warp >> 2) % kSweepChunks;
+    const int q = (warp & 3) * 8 + (lane >> 2), c = lane & 3;
     const uint32_t op_base = sweep_smem(s_op);
-    // a row's operands that do not depend on the level before, in registers
-    double2 b[2][2], dv[2];
+    // a row's operands that do not depend on the levels before, in registers,
+    // and every address its solve needs
+    double2 b[3][2], dv[2];
     double ow = 0.0;
-    int4 r0, tgt;
-    int posb = 0, cnt = 0;
+    int4 r0;
+    bool row = false;
+    uint32_t x0 = 0, x1 = 0, va[4], ba[4];  // operand slots; where the value goes and its barrier (0: nowhere)
+    double* to = nullptr;
     auto load_row = [&](int l) {
       const int slot = l % kStageRing;
       bar_wait(bar_full + 8u * slot, (l / kStageRing) & 1, bad);
       const double* s = s_blk + slot * kStageDoubles + (q * 4 + c) * 2;
       const unsigned char* r = s_rec + (slot * kSweepChunks + j) * kRecChunkBytes + q * (kSweepRec * 4);
-      cnt = s_cnt[slot];
+      const int cnt = s_cnt[slot];
       r0 = *reinterpret_cast<const int4*>(r);
-      tgt = *reinterpret_cast<const int4*>(r + 16);
-      if (kForward) posb = *reinterpret_cast<const int*>(r + 32);
+      const int4 tgt = *reinterpret_cast<const int4*>(r + 16);
+      const int posb = kForward ? *reinterpret_cast<const int*>(r + 32) : 0;
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
         b[d][0] = *reinterpret_cast<const double2*>(s + j * kStageChunkDoubles + d * 512);
@@ -679,37 +708,56 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
         dv[0] = *reinterpret_cast<const double2*>(s + kStageBwdD + j * 512);
         dv[1] = *reinterpret_cast<const double2*>(s + kStageBwdD + j * 512 + 256);
       }
+      row = !bad && j < cnt && r0.x >= 0;  // after a wait that ran out nothing is taken for a record
+      x0 = op_base + ((uint32_t)r0.z & (kSweepSlots - 1)) * 32;
+      x1 = op_base + ((uint32_t)r0.z >> 16 & (kSweepSlots - 1)) * 32;
+      const int tg[4] = {tgt.x, tgt.y, tgt.z, tgt.w};
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const bool on = row && tg[t] >= 0;
+        uint32_t base;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base) : "r"(op_base), "r"(on ? tg[t] >> 16 : rank));
+        va[t] = on ? base + (uint32_t)(tg[t] & 0xfff) * 32 + (uint32_t)c * 8 : 0;
+        ba[t] = base + (bar_op - op_base) + (uint32_t)(tg[t] >> 12 & 15) * 8;
+      }
+      if (r0.y > 2) {  // rare on triangles
+        b[2][0] = *reinterpret_cast<const double2*>(s + j * kStageChunkDoubles + 1024);
+        b[2][1] = *reinterpret_cast<const double2*>(s + j * kStageChunkDoubles + 1024 + 256);
+      }
+      to = !row       ? nullptr
+           : kForward ? reinterpret_cast<double*>(ilu.own_b) + (int64_t)posb * 4 + c
+                      : reinterpret_cast<double*>(z) + (int64_t)r0.x * 4 + c;
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar_empty + 8u * slot);
     };
-    load_row(0);
-    for (int l = 0; l < nlev; ++l) {
-      keep_together(l);
+    if (set < nlev) load_row(set);
+    for (int pair = 0; pair < nlev; pair += 2) {
+      const int l = pair + set;
+      keep_together(pair);
+      if (l >= nlev) break;  // pair was the last level
       double acc = ow;
       bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
-      const bool mine = !bad && j < cnt && r0.x >= 0;  // after a wait that ran out nothing is taken for a record
-      const int nd = mine ? r0.y : 0;
+      const int nd = row ? r0.y : 0;
       // both usual operands at once, whether the row has them or not
-      auto operand = [&](uint32_t slot, double2& x, double2& y) {
-        const double2* v = reinterpret_cast<const double2*>(s_op + (slot & (kSweepSlots - 1)) * 32);
-        x = v[0];
-        y = v[1];
+      auto operand = [&](uint32_t a, double2& x, double2& y) {
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x.x), "=d"(x.y) : "r"(a) : "memory");
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(y.x), "=d"(y.y) : "r"(a + 16) : "memory");
       };
-      double2 x, y, x1, y1;
-      operand((uint32_t)r0.z, x, y);
-      operand((uint32_t)r0.z >> 16, x1, y1);
+      double2 x, y, xx, yy;
+      operand(x0, x, y);
+      operand(x1, xx, yy);
       const double s0 = b[0][0].x * x.x + b[0][0].y * x.y + b[0][1].x * y.x + b[0][1].y * y.y;
-      const double s1 = b[1][0].x * x1.x + b[1][0].y * x1.y + b[1][1].x * y1.x + b[1][1].y * y1.y;
+      const double s1 = b[1][0].x * xx.x + b[1][0].y * xx.y + b[1][1].x * yy.x + b[1][1].y * yy.y;
       if (nd > 0) acc -= s0;
       if (nd > 1) acc -= s1;
-      if (nd > 2) {  // rare on triangles
-        const double* s = s_blk + (l % kStageRing) * kStageDoubles + j * kStageChunkDoubles + 1024 + (q * 4 + c) * 2;
-        const double2 bx = *reinterpret_cast<const double2*>(s), by = *reinterpret_cast<const double2*>(s + 256);
-        operand((uint32_t)r0.w, x, y);
-        acc -= bx.x * x.x + bx.y * x.y + by.x * y.x + by.y * y.y;
+      if (nd > 2) {
+        operand(op_base + ((uint32_t)r0.w & (kSweepSlots - 1)) * 32, x, y);
+        acc -= b[2][0].x * x.x + b[2][0].y * x.y + b[2][1].x * y.x + b[2][1].y * y.y;
         if (nd > 3) {  // quadrilaterals, at the end of an elimination front
           const int64_t k = info[(int64_t)l * C].x + (int64_t)j * C;
           const double* g = ilu.pack[kDir] + k * 2048 + 1536 + (q * 4 + c) * 2;
           const double2 gx = *reinterpret_cast<const double2*>(g), gy = *reinterpret_cast<const double2*>(g + 256);
-          operand((uint32_t)r0.w >> 16, x, y);
+          operand(op_base + ((uint32_t)r0.w >> 16 & (kSweepSlots - 1)) * 32, x, y);
           acc -= gx.x * x.x + gx.y * x.y + gy.x * y.x + gy.y * y.y;
         }
       }
@@ -720,27 +768,18 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
                      a2 = __shfl_sync(0xffffffffu, acc, g + 2), a3 = __shfl_sync(0xffffffffu, acc, g + 3);
         acc = dv[0].x * a0 + dv[0].y * a1 + dv[1].x * a2 + dv[1].y * a3;
       }
-      if (mine) {
-        const int tg[4] = {tgt.x, tgt.y, tgt.z, tgt.w};
+      if (!bad) {
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          if (tg[t] < 0) break;  // the record's targets come first
-          uint32_t base;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base) : "r"(op_base), "r"(tg[t] >> 16));
-          const uint32_t va = base + (uint32_t)(tg[t] & 0xfff) * 32 + (uint32_t)c * 8;
-          const uint32_t ba = base + (bar_op - op_base) + (uint32_t)(tg[t] >> 12 & 15) * 8;
-          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(va),
-                       "l"(__double_as_longlong(acc)), "r"(ba)
+          if (va[t] == 0) break;  // the record's targets come first
+          asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(va[t]),
+                       "l"(__double_as_longlong(acc)), "r"(ba[t])
                        : "memory");
         }
       }
-      double* to = !mine ? nullptr
-                   : kForward ? reinterpret_cast<double*>(ilu.own_b) + (int64_t)posb * 4 + c
-                              : reinterpret_cast<double*>(z) + (int64_t)r0.x * 4 + c;
-      __syncwarp();
-      if (lane == 0) bar_arrive(bar_empty + 8u * (l % kStageRing));
-      if (l + 1 < nlev) load_row(l + 1);
-      if (to) *to = acc;
+      double* const out = bad ? nullptr : to;
+      if (l + 2 < nlev) load_row(l + 2);
+      if (out) *out = acc;
     }
   }
   __syncwarp();

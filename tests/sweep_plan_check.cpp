@@ -126,7 +126,8 @@ struct Bar {
 
 static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<int32_t>& nbr,
                      const std::vector<int32_t>& pos, std::mt19937& rng) {
-  constexpr int kRing = 4, kWarps = 4 * kSweepChunks, kAll = kWarps + kSweepChunks + 1;
+  constexpr int kRing = 4, kWarps = 4 * kSweepChunks;  // warps of a level; two sets of them take turns
+  constexpr int kSolve = 2 * kWarps, kAll = kSolve + kRing + 1;
   const int C = pl.cluster, nlev = pl.nlev[dir];
   const auto &info = pl.info[dir], &rec = pl.rec[dir];
   auto in = [&](int l, int b, int f) { return info[((size_t)l * C + b) * 4 + f]; };
@@ -135,8 +136,8 @@ static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<
     std::vector<int> staged;  // level staged in a slot
     std::vector<int32_t> slot;
     Block()
-        : op(kSweepBars, Bar(1)), full(kRing, Bar(kSweepChunks)), empty(kRing, Bar(kWarps)),
-          staged(kRing * kSweepChunks, -1), slot(kSweepSlots, -1) {}
+        : op(kSweepBars, Bar(1)), full(kRing, Bar(1)), empty(kRing, Bar(kWarps)),
+          staged(kRing, -1), slot(kSweepSlots, -1) {}
   };
   std::vector<Block> blk(C);
   struct Flight {
@@ -146,7 +147,7 @@ static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<
   };
   std::vector<Flight> flight;
   struct Actor {  // a warp: level (-1: prologue), step 0 cluster barrier, 1 wait and work, 2 load the next
-    int level = -1, step = 0, arrivals = 0;
+    int level = -1, step = 0, arrivals = 0;  // level: the first of a solving warp's pair, a staging warp's four
   };
   std::vector<Actor> act(C * kAll);
   auto all_arrived = [&](int k) {
@@ -154,11 +155,11 @@ static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<
       if (a.arrivals < k) return false;
     return true;
   };
-  auto stage = [&](int b, int j, int l) {
+  auto stage = [&](int b, int l) {
     if (l >= nlev) return;
     Bar& f = blk[b].full[l % kRing];
     CHECK(f.done == l / kRing);
-    blk[b].staged[(l % kRing) * kSweepChunks + j] = l;
+    blk[b].staged[l % kRing] = l;
     f.arrive(0);
   };
   auto arm = [&](int b, int l) {
@@ -166,6 +167,14 @@ static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<
     Bar& o = blk[b].op[l % kSweepBars];
     CHECK(o.done == l / kSweepBars);
     o.arrive(in(l, b, 3));
+  };
+  auto load = [&](Block& B, int l) {  // a warp takes its rows of a staged level into registers
+    Bar& f = B.full[l % kRing];
+    if (!f.passes(l / kRing)) return false;
+    CHECK(f.done == l / kRing + 1);
+    CHECK(B.staged[l % kRing] == l);
+    B.empty[l % kRing].arrive(0);
+    return true;
   };
   int64_t idle = 0;
   int finished = 0;
@@ -186,28 +195,30 @@ static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<
     Block& B = blk[b];
     if (a.level >= nlev) continue;
     if (a.level < 0) {  // prologue
-      if (w >= kWarps && w < kWarps + kSweepChunks)
-        for (int l = 0; l < kRing; ++l) stage(b, w - kWarps, l);
-      if (w == kWarps + kSweepChunks)
+      if (w >= kSolve && w < kSolve + kRing) stage(b, w - kSolve);
+      if (w == kSolve + kRing)
         for (int l = 0; l < kSweepNear; ++l) arm(b, l);
-      if (w < kWarps && !B.full[0].passes(0)) continue;
+      if (w < kSolve && w / kWarps < nlev && !load(B, w / kWarps)) continue;
       a.level = 0;
       idle = 0;
       continue;
     }
-    const int l = a.level;
+    const int l = a.level + (w < kSolve ? w / kWarps : w < kSolve + kRing ? w - kSolve : 0);
     if (a.step == 0) {
-      if (l % (kSweepSkew / 2) == 0) {
-        if (l > 0 && !all_arrived(l / (kSweepSkew / 2))) continue;
+      if (a.level % (kSweepSkew / 2) == 0) {
+        if (a.level > 0 && !all_arrived(a.level / (kSweepSkew / 2))) continue;
         ++a.arrivals;
       }
       a.step = 1;
+    } else if (l >= nlev) {
+      a.level = nlev;
+      ++finished;
     } else if (a.step == 1) {
-      if (w < kWarps) {
+      if (w < kSolve) {
         Bar& o = B.op[l % kSweepBars];
         if (!o.passes(l / kSweepBars)) continue;
         CHECK(o.done == l / kSweepBars + 1);
-        const int j = w / 4;
+        const int j = w / 4 % kSweepChunks;
         if (j < in(l, b, 1)) {
           const int64_t k = in(l, b, 0) + (int64_t)j * C;
           for (int q = w % 4 * 8; q < w % 4 * 8 + 8; ++q) {
@@ -227,24 +238,19 @@ static void simulate(const SweepPlan& pl, int dir, int64_t n, const std::vector<
             }
           }
         }
-        B.empty[l % kRing].arrive(0);
-      } else if (w < kWarps + kSweepChunks) {
+      } else if (w < kSolve + kRing) {
         if (!B.empty[l % kRing].passes(l / kRing)) continue;
         CHECK(B.empty[l % kRing].done == l / kRing + 1);
-        stage(b, w - kWarps, l + kRing);
+        stage(b, l + kRing);
       } else {
         arm(b, l + kSweepNear);
       }
       a.step = 2;
     } else {
-      if (w < kWarps && l + 1 < nlev) {
-        Bar& f = B.full[(l + 1) % kRing];
-        if (!f.passes((l + 1) / kRing)) continue;
-        CHECK(f.done == (l + 1) / kRing + 1);
-        for (int j = 0; j < kSweepChunks; ++j) CHECK(B.staged[((l + 1) % kRing) * kSweepChunks + j] == l + 1);
-      }
+      if (w < kSolve && l + 2 < nlev && !load(B, l + 2)) continue;
       a.step = 0;
-      if (++a.level == nlev) ++finished;
+      a.level += w < kSolve ? 2 : w < kSolve + kRing ? kRing : 1;
+      if (a.level >= nlev) a.level = nlev, ++finished;
     }
     idle = 0;
   }
@@ -293,7 +299,7 @@ int main() {
       CHECK(pl.cluster <= kSweepMaxCluster);
       for (int dir = 0; dir < 2; ++dir) {
         walk(pl, dir, n, nbr, pos);
-        if (n <= 5000 && cluster != 1) simulate(pl, dir, n, nbr, pos, rng);
+        if (n <= 5000 && cluster >= 0) simulate(pl, dir, n, nbr, pos, rng);
       }
     }
   }
