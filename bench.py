@@ -595,7 +595,10 @@ def run_candidates(args, rank: int, world: int) -> dict | None:
     if e2e:
         line["e2e"] = e2e
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        line["cpu_baseline"] = cpu_baseline(args, cands[0], rk, plain_out[0]["iters"])
+        try:
+            line["cpu_baseline"] = cpu_baseline(args, cands[0], rk, plain_out[0]["iters"])
+        except FileNotFoundError as err:  # the line stands without it
+            line["cpu_baseline"] = {"unavailable": str(err)}
     return line if rank == 0 else None
 
 
@@ -668,7 +671,7 @@ def reference_eval(c: Candidate, steps: int, iters: int, threads: int) -> dict:
     timed by phase inside the process (the mesh build is not timed)."""
     from oracle import ref
     if not ref.EXE_FAST.exists():
-        raise RuntimeError("reference build oracle/_ref is not present")
+        raise FileNotFoundError("reference build oracle/_ref is not present")
     with tempfile.TemporaryDirectory() as td:
         td = Path(td)
         ref.write_binary_mesh(td / "mesh.bin", c.mesh)
@@ -788,7 +791,10 @@ def main() -> int:
         torch.distributed.init_process_group("nccl", timeout=datetime.timedelta(seconds=1800))
     try:
         if args.impl == "reference":
-            line = run_reference(args, rank, world)
+            try:
+                line = run_reference(args, rank, world)
+            except FileNotFoundError as err:
+                line = {"impl": "reference", "unavailable": str(err)}
         elif args.workload == "large":
             line = run_large(args, rank, world)
         elif args.workload == "kernels":
