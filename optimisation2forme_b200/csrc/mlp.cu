@@ -129,12 +129,9 @@ Mlp::Mlp(int max_batch, float freq_scale, uint64_t seed, cudaStream_t stream)
     : max_batch_(max_batch), stream_(stream) {
   if (max_batch < 128 || max_batch > (1 << 20)) throw Error(O2F_ERR_ARG, "max_batch out of range [128, 2^20]");
   if (!(freq_scale > 0.f)) throw Error(O2F_ERR_ARG, "freq_scale must be positive");
-  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                gemm_smem_bytes<64>()));
-  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                gemm_smem_bytes<64>()));
-  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                gemm_smem_bytes<16>()));
+  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<64>()));
+  O2F_CUDA(cudaFuncSetAttribute(k_gemm_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem_bytes<16>()));
+  O2F_CUDA(cudaFuncSetAttribute(k_weight_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
   // parameter layout: W0, b0, W1, b1, ..., W4, b4
   int64_t off = 0;
   for (int l = 0; l <= kHidden; ++l) {
@@ -210,7 +207,8 @@ Mlp::~Mlp() {
     if (e) cudaEventDestroy(e);
   for (auto& e : fork_)
     if (e) cudaEventDestroy(e);
-  if (join_) cudaEventDestroy(join_);
+  for (auto& e : join_)
+    if (e) cudaEventDestroy(e);
   for (auto& c : capture_)
     if (c) cudaStreamDestroy(c);
   if (slots_) {
@@ -244,33 +242,31 @@ void Mlp::forward(int n, float* y, int outputs, cudaStream_t s) {
       a.out = A_[l];
       a.pre = Z_[l];
       a.ldo = kWidth;
-      k_gemm_tc<64, false>
-          <<<dim3(blocks_of(n, kTileM), blocks_of(a.N, 64)), gemm_threads(64), gemm_smem_bytes<64>(), s>>>(a);
+      k_gemm_tc<64><<<dim3(blocks_of(n, kTileM), blocks_of(a.N, 64)), gemm_threads(64), gemm_smem_bytes<64>(), s>>>(a);
       x = A_[l];
     } else {
       a.N = outputs;
       a.epi = kEpiLinear;
       a.out32 = y;
       a.ldo = outputs;
-      k_gemm_tc<16, false><<<dim3(blocks_of(n, kTileM), 1), gemm_threads(16), gemm_smem_bytes<16>(), s>>>(a);
+      k_gemm_tc<16><<<dim3(blocks_of(n, kTileM), 1), gemm_threads(16), gemm_smem_bytes<16>(), s>>>(a);
     }
     ++launches_;
   }
   O2F_CUDA(cudaGetLastError());
 }
 
-// Backward pass from dY_ into grads_ (zeroed here).  The chain of input
+// Backward pass from dY_ into grads_ (zero on entry).  The chain of input
 // gradients runs on s; a layer's weight and bias gradients, which nothing in
-// the chain needs, on side (when it is another stream: a fork per layer and
-// one join).
-void Mlp::backward(int n, cudaStream_t s, cudaStream_t side) {
-  O2F_CUDA(cudaMemsetAsync(grads_, 0, n_params_ * sizeof(float), side));
+// the chain needs, on side[l] (null: on s too).
+void Mlp::backward(int n, cudaStream_t s, const cudaStream_t* side) {
   const bf16* g = dY_;  // gradient w.r.t. the output of layer l
   for (int l = kHidden; l >= 0; --l) {
     const int N = out_dim(l), K = in_dim(l);
-    if (side != s) {
+    const cudaStream_t sl = side ? side[l] : s;
+    if (side) {
       O2F_CUDA(cudaEventRecord(fork_[l], s));
-      O2F_CUDA(cudaStreamWaitEvent(side, fork_[l], 0));
+      O2F_CUDA(cudaStreamWaitEvent(sl, fork_[l], 0));
     }
     // dW_l[n][k] = sum_m g(m, n) below(m, k), db_l[n] = sum_m g(m, n): the
     // batch is the reduction axis
@@ -282,12 +278,13 @@ void Mlp::backward(int n, cudaStream_t s, cudaStream_t side) {
     w.lda = N;
     w.B = l > 0 ? A_[l - 1] : X0_;
     w.ldb = K;
-    w.epi = kEpiAtomic;
     w.out32 = grads_ + w_off_[l];
     w.bias_grad = grads_ + b_off_[l];
     w.ldo = K;
-    k_gemm_tc<64, true><<<dim3(blocks_of(N, kTileM), blocks_of(K, 64), blocks_of(n, kMaxK)), gemm_threads(64),
-                          gemm_smem_bytes<64>(), side>>>(w);
+    w.k_split = weight_grad_split(n);
+    k_weight_grad<<<dim3(blocks_of(N, kTileM), K / kGradN + kBiasBlocks, blocks_of(n, w.k_split)), kGradThreads,
+                    kGradSmem, sl>>>(w);
+    if (side) O2F_CUDA(cudaEventRecord(join_[l], sl));
     ++launches_;
     if (l == 0) break;
     // gradient w.r.t. the layer below's pre-activation: (g W_l) * silu'(Z_{l-1})
@@ -303,15 +300,13 @@ void Mlp::backward(int n, cudaStream_t s, cudaStream_t side) {
     d.out = dZ_[l - 1];  // one per layer: its weight gradient may still be reading it
     d.zprev = Z_[l - 1];
     d.ldo = kWidth;
-    k_gemm_tc<64, false>
+    k_gemm_tc<64>
         <<<dim3(blocks_of(n, kTileM), blocks_of(K, 64)), gemm_threads(64), gemm_smem_bytes<64>(), s>>>(d);
     ++launches_;
     g = dZ_[l - 1];
   }
-  if (side != s) {
-    O2F_CUDA(cudaEventRecord(join_, side));
-    O2F_CUDA(cudaStreamWaitEvent(s, join_, 0));
-  }
+  if (side)
+    for (auto& e : join_) O2F_CUDA(cudaStreamWaitEvent(s, e, 0));
   O2F_CUDA(cudaGetLastError());
 }
 
@@ -350,7 +345,7 @@ void Mlp::train(int steps, int batch, float lr, uint64_t seed, float* loss_hist)
     O2F_CUDA(cudaMallocHost(&slots_, kSlots * slot_ints * sizeof(int)));
     for (auto& e : slot_free_) O2F_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& e : fork_) O2F_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    O2F_CUDA(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
+    for (auto& e : join_) O2F_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (auto& c : capture_) O2F_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
   }
   build_graph(batch, lr);
@@ -383,18 +378,22 @@ void Mlp::build_graph(int batch, float lr) {
     O2F_CUDA(cudaGraphExecDestroy(graph_));
     graph_ = nullptr;
   }
-  cudaStream_t s = capture_[0], side = capture_[1];
+  cudaStream_t s = capture_[0];
+  const cudaStream_t* side = capture_ + 1;  // one per layer
   const StepHead* head = reinterpret_cast<const StepHead*>(step_in_);
   const int* index = step_in_ + sizeof(StepHead) / sizeof(int);
   const int64_t before = launches_;
   cudaGraph_t graph = nullptr;
   O2F_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   try {
+    O2F_CUDA(cudaEventRecord(fork_[0], s));  // the gradients are zeroed beside the forward pass
+    O2F_CUDA(cudaStreamWaitEvent(side[0], fork_[0], 0));
+    O2F_CUDA(cudaMemsetAsync(grads_, 0, n_params_ * sizeof(float), side[0]));
+    O2F_CUDA(cudaEventRecord(join_[0], side[0]));
     load_batch(data_in_, index, batch, s);
     forward(batch, Y_, kOutPad, s);
+    O2F_CUDA(cudaStreamWaitEvent(s, join_[0], 0));
     k_loss<<<blocks_of(batch, 128), 128, 0, s>>>(batch, Y_, data_out_, index, dY_, loss_buf_, head);
-    O2F_CUDA(cudaEventRecord(join_, s));
-    O2F_CUDA(cudaStreamWaitEvent(side, join_, 0));
     backward(batch, s, side);
     k_adam<<<blocks_of(n_params_, 256), 256, 0, s>>>(n_params_, params_, grads_, adam_m_, adam_v_, lr, 0.9f, 0.999f,
                                                      1e-8f, head, layers());
@@ -461,7 +460,8 @@ void Mlp::gradients(const float* inputs, const float* targets, int n, float* gra
   load_batch(in_dev, nullptr, n, stream_);
   forward(n, Y_, kOutPad, stream_);
   k_loss<<<blocks_of(n, 128), 128, 0, stream_>>>(n, Y_, grad_targets_, nullptr, dY_, loss_, nullptr);
-  backward(n, stream_, stream_);
+  O2F_CUDA(cudaMemsetAsync(grads_, 0, n_params_ * sizeof(float), stream_));
+  backward(n, stream_, nullptr);
   sync();
   O2F_CUDA(cudaMemcpy(grads_out, grads_, n_params_ * sizeof(float), cudaMemcpyDeviceToHost));
   if (loss_out) O2F_CUDA(cudaMemcpy(loss_out, loss_, sizeof(float), cudaMemcpyDeviceToHost));

@@ -34,7 +34,7 @@ class Mlp {
   GemmArgs args() const;
   Layers layers() const;
   void forward(int n, float* y, int outputs, cudaStream_t s);
-  void backward(int n, cudaStream_t s, cudaStream_t side);
+  void backward(int n, cudaStream_t s, const cudaStream_t* side);
   void load_batch(const float* inputs_dev, const int* index_dev, int n, cudaStream_t s);
   void build_graph(int batch, float lr);
   float* arena_scratch_in(int64_t n);
@@ -65,8 +65,8 @@ class Mlp {
   // training: pinned copies of step_in_ that the host fills ahead, the step's graph
   static constexpr int kSlots = 4;
   int* slots_ = nullptr;
-  cudaEvent_t slot_free_[kSlots]{}, fork_[5]{}, join_ = nullptr;
-  cudaStream_t capture_[2]{};
+  cudaEvent_t slot_free_[kSlots]{}, fork_[5]{}, join_[5]{};
+  cudaStream_t capture_[6]{};
   cudaGraphExec_t graph_ = nullptr;
   int64_t graph_launches_ = 0;
   int graph_batch_ = 0;

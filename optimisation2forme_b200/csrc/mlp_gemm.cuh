@@ -2,22 +2,35 @@
 // network: D[M x N] = sum_k A(m, k) B(n, k), BF16 operands staged in shared
 // memory, FP32 accumulators in tensor memory (TMEM), fused epilogues.
 //
-// One CTA computes a 128 x NT tile (NT = 64 or 16) over at most kMaxK of K.  The network's layers are small (K = 128 or 256), so a
-// launch is latency: all K chunks of a tile are requested at once
-// (cp.async, 64 of K each, 96 KB at NT = 64), each chunk's tcgen05.mma
-// (M = 128, N = NT, K = 16) are issued by one thread as it arrives, and one
-// commit to an mbarrier (bounded wait) ends them.  NT = 64 rather than the 256
-// of a whole layer: a batch of 4,096 then is 128 CTAs instead of 32, each with
-// a quarter of the epilogue's exponentials, and two fit an SM.  Every 16
-// columns have four warps of their own (8 threads per column), since with
-// four warps for all columns the epilogue took longer than the product.  The
-// weight
-// gradients reduce over the batch: their K is split over blockIdx.z, kMaxK
-// rows each, and added up with vector reductions.
-// Measured on B200 at batch 4,096: a training step 2,250 -> 130 us (host draws
-// and copies of the next batches beside it), a hidden layer's launch about 9 us
-// alone, nearly all of it latency (batch 256: 124 us a step); the prediction
-// of 74,528 rows through the API 2.24 -> 1.0 ms.
+// One CTA computes a 128 x NT tile (NT = 64 or 16).  The network's layers are
+// small (K = 128 or 256), so a launch is latency: all K chunks of a tile are
+// requested at once (cp.async, 64 of K each, 96 KB at NT = 64), each chunk's
+// tcgen05.mma (M = 128, N = NT, K = 16) are issued by one thread as it arrives,
+// and one commit to an mbarrier (bounded wait) ends them.  NT = 64 rather than
+// the 256 of a whole layer: a batch of 4,096 then is 128 CTAs instead of 32,
+// each with a quarter of the epilogue's exponentials, and two fit an SM.  Every
+// 16 columns have four warps of their own (8 threads per column), since with
+// four warps for all columns the epilogue took longer than the product.
+//
+// The weight gradients reduce over the batch (k_weight_grad).  A sum over it is
+// one tensor memory accumulator up to 2,048 rows (weight_grad_split), so that
+// its bits are a function of the batch alone: two such parts meet by an add
+// onto zero, which commutes, and only batches above 4,096 add three and more
+// in the order they come in.  The bias gradients are eight sums of consecutive
+// rows added in order, by blocks of their own in the same launch.  (Slices of
+// 256 rows by atomic adds are faster, 135 us a step at batch 4,096, but no two
+// runs agree, and Adam's near-zero second moments turn last bits into steps of
+// full size: weights 1.6e-4 apart after 60 steps.)  The rows go through a ring
+// of eight chunks, filled by 16 warps and multiplied by a warp of its own; a
+// launch takes 33 us at batch 4,096, about 1 us a chunk, on 22 to 28 SMs,
+// so the layers' launches run side by side.
+//
+// Measured on B200 at batch 4,096: a training step 156 us (host draws and
+// copies of the next batches beside it; 2,250 with blocks of 256 columns, a
+// chunk at a time and launches from the host; 231 with the weight gradients in
+// one queue), at batch 256 113 us, a hidden layer's launch about 9 us alone,
+// nearly all of it latency; the prediction of 74,528 rows through the API
+// 2.24 -> 1.0 ms.
 //
 // Shared memory holds 8 x 16-byte core matrices without swizzle: K-major
 // operands (rows contiguous in K) and MN-major ones (the weight gradients'
@@ -41,8 +54,7 @@ using bf16 = __nv_bfloat16;
 
 constexpr int kTileM = 128;
 constexpr int kKC = 64;          // K elements per shared-memory chunk
-constexpr int kMaxChunks = 4;
-constexpr int kMaxK = kKC * kMaxChunks;  // K elements of one CTA
+constexpr int kMaxChunks = 4;    // of a layer (K = 256)
 constexpr int gemm_threads(int nt) { return 8 * nt; }
 constexpr long long kWaitLimit = 1ll << 26;  // mbarrier polls before giving up
 
@@ -50,15 +62,16 @@ enum Epilogue : int {
   kEpiHidden = 0,   // z = acc + bias -> pre (bf16), act = silu(z) (bf16)
   kEpiLinear = 1,   // out32 = acc + bias (fp32)
   kEpiBackAct = 2,  // out = bf16(acc * silu'(zprev))
-  kEpiAtomic = 3,   // out32 += acc (fp32 atomics; split-K weight gradients)
 };
 
-// K-major operands (kTrans = false): A(m, k) = A[m*lda + k], B(n, k) =
-// B[n*ldb + k].  MN-major: A(m, k) = A[k*lda + m], B(n, k) = B[k*ldb + n].
-// lda, ldb multiples of 8 elements, A and B 16-byte aligned; K a multiple of
-// 16 (kTrans = false) and M, N multiples of 8 (kTrans = true).
+// k_gemm_tc, K-major operands: A(m, k) = A[m*lda + k], B(n, k) = B[n*ldb + k],
+// K a multiple of 16, at most kMaxChunks * kKC.  k_weight_grad, MN-major ones:
+// A(m, k) = A[k*lda + m], B(n, k) = B[k*ldb + n], M a multiple of 8, N of 64, K
+// any number of rows, k_split of them (a multiple of kKC) per blockIdx.z.
+// lda, ldb, ldo multiples of 8 elements, A and B 16-byte aligned.
 struct GemmArgs {
   int M, N, K;
+  int k_split;        // k_weight_grad
   const bf16* A;
   int64_t lda;
   const bf16* B;
@@ -69,8 +82,8 @@ struct GemmArgs {
   bf16* pre;          // kEpiHidden: pre-activation
   const bf16* zprev;  // kEpiBackAct: pre-activation of the layer below
   int64_t ldo;        // row stride of out / pre / zprev / out32
-  float* out32;       // kEpiLinear / kEpiAtomic
-  float* bias_grad;   // kEpiAtomic: [M] += sum over k of A(m, k)
+  float* out32;       // kEpiLinear; k_weight_grad: += sum over k of A(m, k) B(n, k)
+  float* bias_grad;   // k_weight_grad: [M] = sum over k of A(m, k)
   int* err;           // set when a wait exceeds its limit
 };
 
@@ -149,12 +162,58 @@ __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, fl
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
+// TMEM columns for a block, by one warp; their address goes to slot.
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot, int cols) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t tmem, int cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
+}
+// 16 columns of the warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The products of one chunk (k of its kKC elements hold more than zeros) into
+// tmem, by one thread; first: tmem holds nothing yet.
+template <int NT, bool kTrans>
+__device__ __forceinline__ void multiply_chunk(uint32_t aA, uint32_t aB, int k, uint32_t tmem, bool first) {
+  constexpr auto kMajor = kTrans ? cute::UMMA::Major::MN : cute::UMMA::Major::K;
+  const uint32_t idesc = static_cast<uint32_t>(
+      cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, kTileM, NT, kMajor, kMajor>());
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+  for (int kk = 0; kk < kKC / 16; ++kk) {
+    if (kk * 16 >= k) break;
+    const uint64_t da = kmajor_desc(aA, kTileM, kk), db = kmajor_desc(aB, NT, kk);
+    const uint32_t acc = (first && kk == 0) ? 0u : 1u;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(da), "l"(db), "r"(idesc), "r"(acc)
+        : "memory");
+  }
+}
+// The barrier's phase completes when all products issued so far are complete.
+__device__ __forceinline__ void commit_products(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 template <int NT>
 constexpr int gemm_smem_bytes() {
   return kMaxChunks * (kTileM + NT) * kKC * 2 + 16;
 }
 
-template <int NT, bool kTrans>
+template <int NT>
 __global__ void __launch_bounds__(gemm_threads(NT)) k_gemm_tc(GemmArgs a) {
   constexpr int kThreads = gemm_threads(NT);
   static_assert(NT == 64 || NT == 16, "tile N");
@@ -167,16 +226,14 @@ __global__ void __launch_bounds__(gemm_threads(NT)) k_gemm_tc(GemmArgs a) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * NT;
-  const int kb = blockIdx.z * kMaxK;
-  const int ke = min(a.K, kb + kMaxK);
-  const int chunks = (ke - kb + kKC - 1) / kKC;
+  const int chunks = (a.K + kKC - 1) / kKC;
 
   // every chunk's copies first, one group each
 #pragma unroll
   for (int c = 0; c < kMaxChunks; ++c) {
     if (c < chunks) {
-      fill_chunk<kTileM, kTrans, kThreads>(sA + c * kChunkA, a.A, a.lda, m0, a.M, kb + c * kKC, ke);
-      fill_chunk<NT, kTrans, kThreads>(sB + c * kChunkB, a.B, a.ldb, n0, a.N, kb + c * kKC, ke);
+      fill_chunk<kTileM, false, kThreads>(sA + c * kChunkA, a.A, a.lda, m0, a.M, c * kKC, a.K);
+      fill_chunk<NT, false, kThreads>(sB + c * kChunkB, a.B, a.ldb, n0, a.N, c * kKC, a.K);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
@@ -184,22 +241,13 @@ __global__ void __launch_bounds__(gemm_threads(NT)) k_gemm_tc(GemmArgs a) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(kCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == 0) tmem_alloc(tmem_slot, kCols);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  constexpr auto kMajor = kTrans ? cute::UMMA::Major::MN : cute::UMMA::Major::K;
-  const uint32_t idesc = static_cast<uint32_t>(
-      cute::UMMA::make_instr_desc<cute::bfloat16_t, cute::bfloat16_t, float, kTileM, NT, kMajor, kMajor>());
   const uint32_t aBar = smem_u32(bar);
 
-  float colsum = 0.f;
 #pragma unroll
   for (int c = 0; c < kMaxChunks; ++c) {
     if (c >= chunks) break;
@@ -209,54 +257,23 @@ __global__ void __launch_bounds__(gemm_threads(NT)) k_gemm_tc(GemmArgs a) {
     if (c == 3) asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // smem writes -> tensor core
     __syncthreads();
-    if (threadIdx.x == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t aA = smem_u32(sA + c * kChunkA), aB = smem_u32(sB + c * kChunkB);
-#pragma unroll
-      for (int kk = 0; kk < kKC / 16; ++kk) {
-        if (kb + c * kKC + kk * 16 >= ke) break;  // only zeros from here
-        const uint64_t da = kmajor_desc(aA, kTileM, kk), db = kmajor_desc(aB, NT, kk);
-        const uint32_t acc = (c > 0 || kk > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-            "l"(da), "l"(db), "r"(idesc), "r"(acc)
-            : "memory");
-      }
-    }
-    if (kTrans && blockIdx.y == 0 && a.bias_grad) {  // column sums of A beside the products
-      constexpr int kPart = kKC * kTileM / kThreads;  // of a row's K elements per thread
-      const int m = threadIdx.x % kTileM, k0 = threadIdx.x / kTileM * kPart;
-      const uint8_t* col = sA + c * kChunkA + (m >> 3) * 128 + (m & 7) * 2;
-#pragma unroll
-      for (int k = k0; k < k0 + kPart; ++k)
-        colsum += __bfloat162float(*reinterpret_cast<const bf16*>(col + (k >> 3) * (kTileM / 8) * 128 + (k & 7) * 16));
-    }
+    if (threadIdx.x == 0)
+      multiply_chunk<NT, false>(smem_u32(sA + c * kChunkA), smem_u32(sB + c * kChunkB), a.K - c * kKC, tmem, c == 0);
   }
-  if (threadIdx.x == 0)
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(aBar) : "memory");
+  if (threadIdx.x == 0) commit_products(aBar);
   const bool ok = __syncthreads_and(mbar_wait(aBar, 0));
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   if (!ok) {
     if (threadIdx.x == 0) atomicExch(a.err, 1);
     mbar_wait(aBar, 0);  // the products may still be in flight: one more bounded wait
   } else {
-    if (kTrans && blockIdx.y == 0 && a.bias_grad && m0 + (int)threadIdx.x % kTileM < a.M)
-      atomicAdd(a.bias_grad + m0 + threadIdx.x % kTileM, colsum);
     // Epilogue: warp w owns TMEM lanes (tile rows) 32 (w % 4) .. + 31 of the
     // columns 16 (w / 4) .. + 15.
     const int row = m0 + (warp & 3) * 32 + lane;
     for (int c0 = 16 * (warp >> 2); c0 < NT; c0 += kThreads / 8) {
       uint32_t r[16];
       const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-          "%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-            "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      tmem_ld16(taddr, r);
       if (row >= a.M) continue;
       const int nb = n0 + c0;
       const int64_t o0 = (int64_t)row * a.ldo + nb;
@@ -291,13 +308,6 @@ __global__ void __launch_bounds__(gemm_threads(NT)) k_gemm_tc(GemmArgs a) {
         pg[1] = reinterpret_cast<const uint4*>(gb)[1];
         continue;
       }
-      if (a.epi == kEpiAtomic && nb + 16 <= a.N && (a.ldo & 3) == 0) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 4)
-          red_add4(a.out32 + o0 + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                   __uint_as_float(r[j + 3]));
-        continue;
-      }
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int n = nb + j;
@@ -310,17 +320,171 @@ __global__ void __launch_bounds__(gemm_threads(NT)) k_gemm_tc(GemmArgs a) {
           a.out[o] = __float2bfloat16_rn(silu(z));
         } else if (a.epi == kEpiLinear) {
           a.out32[o] = acc + (a.bias ? a.bias[n] : 0.f);
-        } else if (a.epi == kEpiBackAct) {
-          a.out[o] = __float2bfloat16_rn(acc * silu_grad(__bfloat162float(a.zprev[o])));
         } else {
-          atomicAdd(a.out32 + o, acc);
+          a.out[o] = __float2bfloat16_rn(acc * silu_grad(__bfloat162float(a.zprev[o])));
         }
       }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+  if (warp == 0) tmem_dealloc(tmem, kCols);
+}
+
+// ---------------------------------------------------------------------------
+// Weight gradients: out32[m][n] += sum over the batch of A(m, k) B(n, k).
+
+constexpr int kGradN = 64;                      // columns of a tile
+constexpr int kGradLoaders = 512;               // threads that copy operands and write the tile
+constexpr int kGradThreads = kGradLoaders + 32; // and a warp that issues the products
+constexpr int kGradRing = 8;                    // chunks in shared memory
+constexpr int kGradLag = 3;                     // of them on their way
+static_assert(kGradLag < kGradRing, "a slot is free only after its products");
+constexpr int kGradSmem = kGradRing * ((kTileM + kGradN) * kKC * 2 + 16) + 16;
+constexpr int kBiasSlices = 8;
+constexpr int kBiasBlocks = 4;  // blocks that compute the bias gradients of a tile's rows
+constexpr int kBiasRows = kTileM / kBiasBlocks;
+static_assert(kBiasSlices * kBiasRows / 2 <= kGradThreads, "a thread per pair of rows and slice");
+
+// Rows of the batch that one accumulator adds up.
+inline int weight_grad_split(int n) {
+  const int splits = n > 64 * 2048 ? 64 : (n + 2047) / 2048;
+  return ((n + splits - 1) / splits + kKC - 1) / kKC * kKC;
+}
+
+// Bias gradients of rows m0 .. m0 + kBiasRows - 1 of A: kBiasSlices sums of
+// consecutive k, each by one thread in order, then added up in order.  A
+// thread sums two neighbouring rows.  (More rows a block: bound by what one SM
+// can read.)
+__device__ __forceinline__ void bias_grad_rows(const GemmArgs& a, int m0, float* part) {
+  constexpr int kAhead = 64;
+  const int slice = threadIdx.x / (kBiasRows / 2), m = threadIdx.x % (kBiasRows / 2) * 2;
+  const int per = (a.K + kBiasSlices - 1) / kBiasSlices;
+  const int k1 = min(a.K, (slice + 1) * per);
+  float s0 = 0.f, s1 = 0.f;
+  if (slice < kBiasSlices && m0 + m < a.M) {
+    const bf16* p = a.A + m0 + m;
+    auto row = [&](int k) { return *reinterpret_cast<const __nv_bfloat162*>(p + (int64_t)k * a.lda); };
+    int k = slice * per;
+    for (; k + kAhead <= k1; k += kAhead) {
+      __nv_bfloat162 v[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) v[u] = row(k + u);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        s0 += __low2float(v[u]);
+        s1 += __high2float(v[u]);
+      }
+    }
+    for (; k < k1; ++k) {
+      const __nv_bfloat162 v = row(k);
+      s0 += __low2float(v);
+      s1 += __high2float(v);
+    }
+  }
+  if (slice < kBiasSlices) {
+    part[slice * kBiasRows + m] = s0;
+    part[slice * kBiasRows + m + 1] = s1;
+  }
+  __syncthreads();
+  if (threadIdx.x < kBiasRows && m0 + (int)threadIdx.x < a.M) {
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < kBiasSlices; ++q) t += part[q * kBiasRows + threadIdx.x];
+    a.bias_grad[m0 + threadIdx.x] = t;
+  }
+}
+
+__global__ void __launch_bounds__(kGradThreads) k_weight_grad(GemmArgs a) {
+  constexpr int kChunkA = kTileM * kKC * 2, kChunkB = kGradN * kKC * 2;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int m0 = blockIdx.x * kTileM;
+  if (blockIdx.y * kGradN >= a.N) {  // kBiasBlocks of them
+    if (blockIdx.z == 0)
+      bias_grad_rows(a, m0 + (blockIdx.y - a.N / kGradN) * kBiasRows, reinterpret_cast<float*>(smem));
+    return;
+  }
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + kGradRing * kChunkA;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sB + kGradRing * kChunkB);  // a slot's copies have arrived
+  uint64_t* done = full + kGradRing;                                       // its products are complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + kGradRing);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.y * kGradN;
+  const int kb = blockIdx.z * a.k_split;
+  const int ke = min(a.K, kb + a.k_split);
+  const int chunks = (ke - kb + kKC - 1) / kKC;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kGradRing; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(full + i)), "r"(kGradLoaders / 32)
+                   : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(done + i)) : "memory");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tmem_alloc(tmem_slot, kGradN);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  // the n-th use of a slot: chunk n * kGradRing + slot
+  auto wait_done = [&](int c) { return mbar_wait(smem_u32(done + c % kGradRing), (uint32_t)(c / kGradRing) & 1u); };
+  bool ok = true;
+  if (threadIdx.x < kGradLoaders) {
+    // one lane of a warp waits and arrives for it
+    for (int c = 0; c < chunks + kGradLag; ++c) {
+      if (c < chunks) {
+        if (c >= kGradRing) {
+          if (lane == 0) ok = wait_done(c - kGradRing);
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          if (!ok) break;
+        }
+        const int slot = c % kGradRing;
+        fill_chunk<kTileM, true, kGradLoaders>(sA + slot * kChunkA, a.A, a.lda, m0, a.M, kb + c * kKC, ke);
+        fill_chunk<kGradN, true, kGradLoaders>(sB + slot * kChunkB, a.B, a.ldb, n0, a.N, kb + c * kKC, ke);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if (c < kGradLag) continue;
+      asm volatile("cp.async.wait_group %0;" ::"n"(kGradLag) : "memory");  // chunk c - kGradLag is there
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(full + (c - kGradLag) % kGradRing))
+                     : "memory");
+    }
+    if (ok && lane == 0) ok = wait_done(chunks - 1);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (threadIdx.x == kGradLoaders) {
+    int c = 0;
+    for (; c < chunks; ++c) {
+      const int slot = c % kGradRing;
+      ok = mbar_wait(smem_u32(full + slot), (uint32_t)(c / kGradRing) & 1u);
+      if (!ok) break;
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // smem writes -> tensor core
+      multiply_chunk<kGradN, true>(smem_u32(sA + slot * kChunkA), smem_u32(sB + slot * kChunkB), ke - kb - c * kKC,
+                                   tmem, c == 0);
+      commit_products(smem_u32(done + slot));
+    }
+    if (c > 0 && !wait_done(c - 1)) ok = false;  // none in flight when the block ends
+  }
+  ok = __syncthreads_and(ok);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!ok) {
+    if (threadIdx.x == 0) atomicExch(a.err, 1);
+  } else if (threadIdx.x < kGradLoaders) {
+    const int row = m0 + (warp & 3) * 32 + lane, c0 = 16 * (warp >> 2);
+    uint32_t r[16];
+    tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, r);
+    if (row < a.M) {
+      float* out = a.out32 + (int64_t)row * a.ldo + n0 + c0;
+#pragma unroll
+      for (int j = 0; j < 16; j += 4)
+        red_add4(out + j, __uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                 __uint_as_float(r[j + 3]));
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, kGradN);
 }
 
 }  // namespace mlp
