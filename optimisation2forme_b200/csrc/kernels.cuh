@@ -320,7 +320,7 @@ __device__ __forceinline__ VertexFan<T> vertex_fan(int64_t v, const int32_t* __r
 
 template <typename T>
 __device__ __forceinline__ Vec4<T> vertex_state_of(const VertexFan<T>& f, const int32_t* __restrict__ vcid,
-                                                   const T* __restrict__ vw, const Vec4<T>* __restrict__ U,
+                                                   const T* __restrict__ vw, const Vec4<T>* U,
                                                    const Phys& ph) {
   T a = (T)0.0, b = (T)0.0, c = (T)0.0, d = (T)0.0;
 #pragma unroll
@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(kBlock) k_vertex_state(int64_t nv, const int32
 // far field and wall vertices are zeroed.
 template <typename T>
 __device__ __forceinline__ Vec4<T> vertex_visc_of(const VertexFan<T>& f, const int32_t* __restrict__ vcid,
-                                                  const T* __restrict__ vw, const Vec4<T>* __restrict__ ctq,
-                                                  const T* __restrict__ ctqy, T& qy) {
+                                                  const T* __restrict__ vw, const Vec4<T>* ctq,
+                                                  const T* ctqy, T& qy) {
   T a = (T)0.0, b = (T)0.0, c = (T)0.0, d = (T)0.0, e = (T)0.0;
 #pragma unroll
   for (int h = 0; h < kFan; h += 4) {
@@ -508,9 +508,9 @@ struct EdgeVertexStates {
 template <typename T, bool kWriteGrad, bool kPlain, int kAlpha = 0, typename VQ>
 __device__ __forceinline__ bool cell_gradient_body(int64_t c,
     int64_t nc, const int32_t* __restrict__ slot, Geom<T> g, VQ vq,
-    const int2* __restrict__ ec, const uint8_t* __restrict__ ebc, const Vec4<T>* __restrict__ U,
-    Phys ph, Vec4<T>* __restrict__ eL, Vec4<T>* __restrict__ eR,
-    Vec4<T>* __restrict__ ctq, T* __restrict__ ctqy, Vec4<T>* __restrict__ grad, Vec4<T>* __restrict__ alpha = nullptr) {
+    const int2* __restrict__ ec, const uint8_t* __restrict__ ebc, const Vec4<T>* U,
+    Phys ph, Vec4<T>* eL, Vec4<T>* eR,
+    Vec4<T>* ctq, T* ctqy, Vec4<T>* grad, Vec4<T>* alpha = nullptr) {
   const Vec4<T> cg = g.cgeom[c];
   const T cx = cg.a, cy = cg.b, cv = cg.c, veps = cg.d;
   const Vec4<T> u = U[c];
@@ -682,19 +682,19 @@ __device__ __forceinline__ bool cell_gradient_body(int64_t c,
 template <typename T, bool kWriteGrad, int kAlpha = 0, typename VQ>
 __device__ __noinline__ void cell_gradient_plain(int64_t c,
     int64_t nc, const int32_t* __restrict__ slot, Geom<T> g, VQ vq,
-    const int2* __restrict__ ec, const uint8_t* __restrict__ ebc, const Vec4<T>* __restrict__ U,
-    Phys ph, Vec4<T>* __restrict__ eL, Vec4<T>* __restrict__ eR,
-    Vec4<T>* __restrict__ ctq, T* __restrict__ ctqy, Vec4<T>* __restrict__ grad, Vec4<T>* __restrict__ alpha) {
+    const int2* __restrict__ ec, const uint8_t* __restrict__ ebc, const Vec4<T>* U,
+    Phys ph, Vec4<T>* eL, Vec4<T>* eR,
+    Vec4<T>* ctq, T* ctqy, Vec4<T>* grad, Vec4<T>* alpha) {
   cell_gradient_body<T, kWriteGrad, true, kAlpha>(c, nc, slot, g, vq, ec, ebc, U, ph, eL, eR, ctq, ctqy, grad, alpha);
 }
 
 template <typename T, bool kWriteGrad, int kAlpha = 0, typename VQ>
 __device__ __forceinline__ void cell_gradient_from(int64_t c,
     int64_t nc, const int32_t* __restrict__ slot, Geom<T> g, VQ vq,
-    const int2* __restrict__ ec, const uint8_t* __restrict__ ebc, const Vec4<T>* __restrict__ U,
-    Phys ph, Vec4<T>* __restrict__ eL, Vec4<T>* __restrict__ eR,
-    Vec4<T>* __restrict__ ctq, T* __restrict__ ctqy, Vec4<T>* __restrict__ grad,
-    Vec4<T>* __restrict__ alpha = nullptr) {
+    const int2* __restrict__ ec, const uint8_t* __restrict__ ebc, const Vec4<T>* U,
+    Phys ph, Vec4<T>* eL, Vec4<T>* eR,
+    Vec4<T>* ctq, T* ctqy, Vec4<T>* grad,
+    Vec4<T>* alpha = nullptr) {
   if (!cell_gradient_body<T, kWriteGrad, false, kAlpha>(c, nc, slot, g, vq, ec, ebc, U, ph, eL, eR, ctq, ctqy, grad,
                                                         alpha))
     cell_gradient_plain<T, kWriteGrad, kAlpha>(c, nc, slot, g, vq, ec, ebc, U, ph, eL, eR, ctq, ctqy, grad, alpha);
@@ -899,8 +899,8 @@ __device__ __noinline__ Vec4<T> cell_residual_plain(int64_t c, int64_t nc, const
 template <typename T, bool kRk, typename ED>
 __device__ __forceinline__ double cell_residual_from(int64_t c, int64_t nc, const int32_t* __restrict__ slot,
                                                      const Vec4<T>* __restrict__ cgeom, ED ed,
-                                                     Vec4<T>* __restrict__ U, Vec4<T>* __restrict__ Uold,
-                                                     Vec4<T>* __restrict__ R, const RkStage& rk,
+                                                     Vec4<T>* U, Vec4<T>* Uold,
+                                                     Vec4<T>* R, const RkStage& rk,
                                                      Vec4<T>* unew = nullptr) {
   double r2 = 0.0;
   Vec4<T> u = U[c], r;

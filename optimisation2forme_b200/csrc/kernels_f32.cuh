@@ -40,9 +40,9 @@ __device__ __forceinline__ double stage_update(const RkStage& rk, double uo, dou
 template <bool kRk, typename ED>
 __device__ __forceinline__ double cell_residual_mixed_from(
     int64_t c, int64_t nc, const int32_t* __restrict__ slot, const Vec4<float>* __restrict__ cgeom, ED ed,
-    Vec4<float>* __restrict__ U32,
-    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, Vec4<double>* __restrict__ R, const RkStage& rk,
-    const double* dtp, Vec4<double>* __restrict__ keep, Vec4<double>* unew = nullptr) {
+    Vec4<float>* U32,
+    Vec4<double>* U, Vec4<double>* Uold, Vec4<double>* R, const RkStage& rk,
+    const double* dtp, Vec4<double>* keep, Vec4<double>* unew = nullptr) {
   double r2 = 0.0;
   const float cv = cgeom[c].c;
   int sl[4], nk = 0;

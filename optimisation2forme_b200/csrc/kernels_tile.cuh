@@ -99,7 +99,12 @@ inline size_t tile_residual_smem(const TileDev& td) {
 // Programmatic dependent launch: the next kernel of the step may start as
 // soon as this one's blocks have all started, and does what depends on the
 // mesh alone (index chains, geometry into L1) before step_inputs() waits for
-// this one's results.
+// this one's results.  What the step's kernels write (states, interface
+// states, viscous terms, residuals) is therefore not constant while a kernel
+// that reads it runs: neither the tile kernels nor the device functions they
+// share with the separate kernels take it as __restrict__, which would let its
+// loads go round the coherent path, or ahead of the wait.  The mesh's arrays
+// are constant and do.
 __device__ __forceinline__ void step_inputs() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -110,7 +115,7 @@ __device__ __forceinline__ void warm_l1(const void* p) { asm volatile("prefetch.
 // global memory (a vertex of several tiles gets the same value from each).
 template <typename T>
 __device__ __forceinline__ void tile_gradient(int tile, const TileDev& td, const Topo& t, const Geom<T>& g,
-                                              const Vec4<T>* __restrict__ U, const Phys& ph, const Work<T>& w,
+                                              const Vec4<T>* U, const Phys& ph, const Work<T>& w,
                                               Vec4<T>* vq_out, Vec4<T>* s_vq, const int* gate) {
   const int v0 = td.voff[tile], nv = td.voff[tile + 1] - v0;
   const int64_t c = (int64_t)tile * td.cells + threadIdx.x;
@@ -247,7 +252,7 @@ __device__ __forceinline__ void tile_stage_end(int tiles, double* part, double* 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kTileMax, 4) k_tile_gradient(TileDev td, Topo t, Geom<T> g, const Vec4<T>* __restrict__ U,
+__global__ void __launch_bounds__(kTileMax, 4) k_tile_gradient(TileDev td, Topo t, Geom<T> g, const Vec4<T>* U,
                                                              Phys ph, Work<T> w, Vec4<T>* vq_out, const int* gate) {
   extern __shared__ __align__(32) unsigned char tile_sm[];
   tile_gradient<T>(blockIdx.x, td, t, g, U, ph, w, vq_out, reinterpret_cast<Vec4<T>*>(tile_sm), gate);
@@ -256,8 +261,8 @@ __global__ void __launch_bounds__(kTileMax, 4) k_tile_gradient(TileDev td, Topo 
 // FP64: residual and update of the state.
 template <int kStage>
 __global__ void __launch_bounds__(kTileMax, 4) k_tile_residual(TileDev td, Topo t, Geom<double> g, Phys ph,
-                                                             Work<double> w, Vec4<double>* __restrict__ U,
-                                                             Vec4<double>* __restrict__ Uold, RkStage rk, double* part,
+                                                             Work<double> w, Vec4<double>* U,
+                                                             Vec4<double>* Uold, RkStage rk, double* part,
                                                              double* hist, StepState* st) {
   extern __shared__ __align__(32) unsigned char tile_sm[];
   const int64_t c = (int64_t)blockIdx.x * td.cells + threadIdx.x;

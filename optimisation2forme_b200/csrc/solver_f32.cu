@@ -95,8 +95,8 @@ void batch_launch_mixed(int phase, bool rk, const RkStage& stage, bool keep, con
 // FP32 residual, update of the FP64 state and its FP32 shadow.
 template <int kStage>
 __global__ void __launch_bounds__(kTileMax, 4) k_tile_residual_mixed(
-    TileDev td, Topo t, Geom<float> g, Phys ph, Work<float> w, Vec4<float>* __restrict__ U32,
-    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, RkStage rk, Vec4<double>* __restrict__ keep,
+    TileDev td, Topo t, Geom<float> g, Phys ph, Work<float> w, Vec4<float>* U32,
+    Vec4<double>* U, Vec4<double>* Uold, RkStage rk, Vec4<double>* keep,
     double* part, double* hist, StepState* st) {
   extern __shared__ __align__(32) unsigned char tile_sm[];
   const int64_t c = (int64_t)blockIdx.x * td.cells + threadIdx.x;
