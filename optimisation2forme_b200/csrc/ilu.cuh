@@ -535,12 +535,13 @@ __device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Whether the phase has completed; sleeps up to a microsecond for it.
+// Whether the phase has completed; sleeps up to a microsecond for it.  Acquire
+// at cluster scope: the values it counts come from other blocks (st.async).
 __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(bar), "r"(parity), "r"(1000)
