@@ -463,10 +463,10 @@ constexpr int kL2Lead = 16;         // levels between the L2 prefetch of a level
 constexpr int kSweepBlockBytes = kStageRing * kStageDoubles * 8;
 constexpr int kSweepOwnBytes = kStageRing * kStageOwn * 8;
 constexpr int kSweepRecBytes = kStageRing * kSweepChunks * kRecChunkBytes;
-// operand slots, blocks, own values + records + mbarriers + chunk counts
-constexpr size_t kSweepSmem = sizeof(Vec4<double>) * kSweepWindow + 4 * kStageDoubles * sizeof(double) + 20688;
+// operand slots, blocks, own values + records + mbarriers + chunk counts + the mark of a wait that ran out
+constexpr size_t kSweepSmem = sizeof(Vec4<double>) * kSweepWindow + 4 * kStageDoubles * sizeof(double) + 20692;
 static_assert(kSweepSmem == 32 * kSweepWindow + kSweepBlockBytes + kSweepOwnBytes + kSweepRecBytes +
-                                8 * (kSweepBars + 2 * kStageRing) + 4 * kStageRing,
+                                8 * (kSweepBars + 2 * kStageRing) + 4 * kStageRing + 4,
               "shared memory of a sweep block");
 static_assert(kSweepSmem <= 227 * 1024, "block sweep shared memory above the per-block limit");
 static_assert(kStageBwdD + kStageChunksBwd * 512 <= kStageDoubles, "backward staging overflows its buffer");
@@ -548,25 +548,36 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait for the phase of an mbarrier; once one has run out (bad), none
-// waits any more.
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, bool& bad) {
-  if (bad) return;
-  for (int i = 0; i < kSweepWaitLimit; ++i)
-    if (bar_try(bar, parity)) return;
-  bad = true;
-}
+// Bounded wait for the phase of an mbarrier.  When one has run out (bad), the
+// warp waits no more, and the block's other warps give up at their next wait
+// that is not over at once (quit).
+struct SweepWaits {
+  int limit;           // polls
+  volatile int* quit;  // in shared memory
+  bool bad;
+  __device__ __forceinline__ void operator()(uint32_t bar, uint32_t parity) {
+    if (bad || bar_try(bar, parity)) return;
+    for (int i = 0; i < limit && !*quit; ++i)
+      if (bar_try(bar, parity)) return;
+    bad = true;
+    *quit = 1;
+  }
+};
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
 // r (in forward sweep order, ilu.own_f) -> ilu.own_b (kForward), ilu.own_b ->
-// z (backward).  Grid: one cluster.  Every wait on an mbarrier is bounded;
-// when one runs out the sweep records sync->err, waits on none any more, uses
-// nothing it waited for, and still takes part in every cluster barrier.
+// z (backward).  Grid: one cluster.  Every wait on an mbarrier is bounded
+// (ilu.spin_limit).  A warp whose wait runs out waits on none any more, uses
+// nothing it waited for, tells nobody that it has read a staged slot (which is
+// then never filled again under a warp that still reads it), sends no values,
+// and still takes part in every cluster barrier; warps that need what it held
+// back run out too.  At the end it records sync->err, and the sweeps after
+// that return at once (their input is void).
 template <bool kForward>
 __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev ilu, Vec4<double>* z, const int* gate) {
-  if (gated(gate)) return;
+  if ((int)gated(gate) | ilu.sync[0].err | ilu.sync[1].err) return;  // (loaded side by side)
   constexpr int kDir = kForward ? 0 : 1;
   extern __shared__ __align__(128) unsigned char sweep_sm[];
   double* s_blk = reinterpret_cast<double*>(sweep_sm);
@@ -577,6 +588,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
   const uint32_t bar_full = bar_op + 8 * kSweepBars;           // staged copies of a level
   const uint32_t bar_empty = bar_full + 8 * kStageRing;        // its last reader
   int* s_cnt = reinterpret_cast<int*>(s_rec + kSweepRecBytes + 8 * (kSweepBars + 2 * kStageRing));
+  int* s_quit = s_cnt + kStageRing;
   const int nlev = ilu.cl_nlev[kDir];
   const int C = (int)gridDim.x, rank = (int)blockIdx.x;
   const int4* __restrict__ info = reinterpret_cast<const int4*>(ilu.cl_info[kDir]) + rank;
@@ -587,11 +599,14 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       bar_init(bar_full + 8u * i, 1);
       bar_init(bar_empty + 8u * i, kSweepWarps);
     }
+    *s_quit = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // all blocks run, their mbarriers are set up
-  bool bad = false;
+  SweepWaits wait{(int)(ilu.spin_limit < kSweepWaitLimit ? ilu.spin_limit : kSweepWaitLimit), s_quit, false};
+  const bool& bad = wait.bad;
+  int staged = -1;  // the level that the thread's copies were started for last
   // Before level 4 i a warp arrives for the i-th time, once all have arrived
   // for the (i-1)-th: at level l every level up to l - kSweepSkew has been
   // left.  (Relaxed: what a warp read of those levels it has used by then.)
@@ -613,8 +628,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
     auto info_of = [&](int l) { return l < nlev ? info[(int64_t)l * C] : make_int4(0, -1, 0, 0); };
     if (slot < kStageRing) {
       const uint32_t bar = bar_full + 8u * slot;
-      auto stage = [&](const int4& in) {
+      auto stage = [&](int l, const int4& in) {
         if (in.y < 0) return;
+        staged = l;
         s_cnt[slot] = in.y;
         uint32_t bytes = 0;
         for (int j = 0; j < in.y; ++j)
@@ -632,7 +648,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       };
       int4 next{};
       if (lane == 0) {
-        stage(info_of(slot));
+        stage(slot, info_of(slot));
         next = info_of(slot + kStageRing);
       }
       for (int l = slot; l - slot < nlev; l += kStageRing) {
@@ -640,14 +656,16 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
         if (lane == 0 && l < nlev) {
           const int4 in = next;
           next = info_of(l + 2 * kStageRing);
-          bar_wait(bar_empty + 8u * slot, (l / kStageRing) & 1, bad);
-          if (!bad) stage(in);
+          wait(bar_empty + 8u * slot, (l / kStageRing) & 1);
+          if (!bad) stage(l + kStageRing, in);
         }
       }
     } else {
       // A level's barrier is set kSweepNear levels ahead: by then every warp
       // has left the level that used it last (kSweepSkew levels back), so a
       // phase that has nothing to wait for cannot pass one that is waited on.
+      // (That level's phase is over then, unless a value was held back: it is
+      // looked at, since a phase must not be set twice.)
       const bool arms = slot == kStageRing;
       const int kLead = arms ? kSweepNear : kL2Lead;
       auto work = [&](int l, const int4& in) {
@@ -673,8 +691,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       for (int l = 0; l < nlev; ++l) {
         keep_together(l);
         const int4 in = entry(l + kLead);
-        if (!arms) bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
-        bad = __any_sync(0xffffffffu, bad);
+        const int last = arms ? l + kSweepNear - kSweepBars : l;
+        if (last >= 0) wait(bar_op + 8u * (last % kSweepBars), (last / kSweepBars) & 1);
+        wait.bad = __any_sync(0xffffffffu, bad);
         if (!bad) work(l + kLead, in);
       }
     }
@@ -692,7 +711,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
     double* to = nullptr;
     auto load_row = [&](int l) {
       const int slot = l % kStageRing;
-      bar_wait(bar_full + 8u * slot, (l / kStageRing) & 1, bad);
+      wait(bar_full + 8u * slot, (l / kStageRing) & 1);
       const double* s = s_blk + slot * kStageDoubles + (q * 4 + c) * 2;
       const unsigned char* r = s_rec + (slot * kSweepChunks + j) * kRecChunkBytes + q * (kSweepRec * 4);
       const int cnt = s_cnt[slot];
@@ -715,7 +734,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       const int tg[4] = {tgt.x, tgt.y, tgt.z, tgt.w};
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const bool on = row && tg[t] >= 0;
+        const bool on = row && tg[t] >= 0 && (!kForward || r0.x != ilu.stall_row);
         uint32_t base;
         asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base) : "r"(op_base), "r"(on ? tg[t] >> 16 : rank));
         va[t] = on ? base + (uint32_t)(tg[t] & 0xfff) * 32 + (uint32_t)c * 8 : 0;
@@ -729,7 +748,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
            : kForward ? reinterpret_cast<double*>(ilu.own_b) + (int64_t)posb * 4 + c
                       : reinterpret_cast<double*>(z) + (int64_t)r0.x * 4 + c;
       __syncwarp();
-      if (lane == 0) bar_arrive(bar_empty + 8u * slot);
+      if (lane == 0 && !bad) bar_arrive(bar_empty + 8u * slot);
     };
     if (set < nlev) load_row(set);
     for (int pair = 0; pair < nlev; pair += 2) {
@@ -737,7 +756,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       keep_together(pair);
       if (l >= nlev) break;  // pair was the last level
       double acc = ow;
-      bar_wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1, bad);
+      wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1);
       const int nd = row ? r0.y : 0;
       // both usual operands at once, whether the row has them or not
       auto operand = [&](uint32_t a, double2& x, double2& y) {
@@ -787,13 +806,17 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
   cluster_wait();
   cluster_arrive();
   cluster_wait();  // no block leaves while another may still write into it
+  // What is on its way into this block's shared memory ends before the block:
+  // its own copies, which a warp that gave up did not wait for, and values of
+  // other blocks, all sent by now, that no warp waited for (a store to
+  // another SM takes microseconds: a millisecond).
+  if (staged >= 0) {
+    for (int i = 0; i < kSweepWaitLimit; ++i)
+      if (bar_try(bar_full + 8u * (staged % kStageRing), (staged / kStageRing) & 1)) break;
+  }
   if (bad) {
     atomicExch(&ilu.sync[kDir].err, 1);
-    // copies of the last levels may still be in flight
-    for (int l = nlev > kStageRing ? nlev - kStageRing : 0; l < nlev; ++l) {
-      bool late = false;
-      bar_wait(bar_full + 8u * (l % kStageRing), (l / kStageRing) & 1, late);
-    }
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
 }
 

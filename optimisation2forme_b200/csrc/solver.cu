@@ -798,15 +798,16 @@ void Solver::ilu_apply(const Vec4<double>* r, Vec4<double>* z, const int* gate) 
   k_ilu_sweep<false><<<blocks, kSweepBlock, 0, s>>>(n, ilu_, nullptr, z, gate);  // ilu_.tmp -> z
 }
 
-// Test hook: the next solves run the waiting sweeps (k_ilu_sweep) with
-// `spin_limit` polls per wait, and with `stall` the first row of the forward order never writes its
-// value, so the rows that depend on it wait out their limit (no fault:
-// every wait is bounded).  spin_limit <= 0 and stall = 0 restore the
+// Test hook: the next solves run with `spin_limit` polls per wait, and with
+// `stall` the first row of the forward order never releases its value, so the
+// rows that depend on it wait out their limit (no fault: every wait is
+// bounded).  stall 2: in the sweeps that the parameters select, else in the
+// waiting ones (k_ilu_sweep).  spin_limit <= 0 and stall = 0 restore the
 // defaults.  Takes effect for the solves that start after the call.
 void Solver::debug_ilu_stall(int stall, long long spin_limit) {
   ilu_.spin_limit = spin_limit > 0 ? spin_limit : kSweepSpinLimit;
   ilu_.stall_row = stall && !ilu_sweep_h_.empty() ? ilu_sweep_h_[0] : -1;
-  ilu_waiting_ = stall != 0 || spin_limit > 0;  // the hook needs the sweeps that wait
+  ilu_waiting_ = stall != 2 && (stall != 0 || spin_limit > 0);
 }
 
 // A sweep whose dependency wait ran out leaves an invalid result: report it

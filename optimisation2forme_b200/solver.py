@@ -548,11 +548,13 @@ class Solver:
         check(lib().o2f_residual_norm_noalloc(self._h, C.byref(out)))
         return out.value
 
-    def debug_ilu_stall(self, stall: bool, spin_limit: int = 0) -> None:
+    def debug_ilu_stall(self, stall: bool, spin_limit: int = 0, selected: bool = False) -> None:
         """Test hook (o2f_debug_ilu_stall): the solves started afterwards run
-        their ILU sweeps with one row that never signals and `spin_limit`
-        polls per wait, so a bounded wait runs out; False / 0 restore."""
-        check(lib().o2f_debug_ilu_stall(self._h, int(bool(stall)), int(spin_limit)))
+        their ILU sweeps with one row that never releases its value and
+        `spin_limit` polls per wait, so a bounded wait runs out; False / 0
+        restore.  `selected`: in the sweeps that adjoint_sweeps selects, not
+        the waiting ones."""
+        check(lib().o2f_debug_ilu_stall(self._h, (2 if selected else 1) if stall else 0, int(spin_limit)))
 
     def timing(self) -> dict:
         t = _lib.Timing()
