@@ -347,8 +347,10 @@ void Solver::upload_mesh() {
   O2F_CUDA(cudaMemsetAsync(ks_, 0, sizeof(KrylovState), s));
   sync();  // host staging vectors go out of scope
   setup_ilu_host(jslot, ec, ebc);
-  slot_h_ = std::move(slot);
-  ev_h_ = std::move(ev);
+  if (tile_cells(nc) > 0) {  // for build_tiles
+    slot_h_ = std::move(slot);
+    ev_h_ = std::move(ev);
+  }
 }
 
 // Geometry of the host mesh in device order: cell centres and volumes, edge
@@ -691,28 +693,6 @@ void Solver::ilu_factor() {
     ilu_.Dinv = arena_.alloc<double>(16 * nc);
     ilu_.order = arena_.alloc<int32_t>(nc);
     ilu_.sweep = arena_.alloc<int32_t>(2 * nc);
-    // made here: a context that only steps in time has no use for it
-    ilu_plan_h_ = make_sweep_plan(nc, ilu_nbr_h_, ilu_pos_h_, ilu_order_h_);
-    const SweepPlan& pl = ilu_plan_h_;
-    if (pl.cluster > 0) {
-      ilu_.cl_blocks = pl.cluster;
-      for (int d = 0; d < 2; ++d) {
-        ilu_.cl_nlev[d] = pl.nlev[d];
-        ilu_.cl_chunks[d] = (int)pl.chunks[d];
-        ilu_.cl_info[d] = arena_.alloc<int32_t>(pl.info[d].size());
-        ilu_.cl_rec[d] = arena_.alloc<int32_t>(pl.rec[d].size());
-        ilu_.pack[d] = arena_.alloc<double>(pl.chunks[d] * 2048);
-        h2d(ilu_.cl_info[d], pl.info[d], s);
-        h2d(ilu_.cl_rec[d], pl.rec[d], s);
-      }
-      ilu_.cl_pos = arena_.alloc<int32_t>(nc);
-      ilu_.packD = arena_.alloc<double>(pl.chunks[1] * 512);
-      ilu_.own_f = arena_.alloc<Vec4<double>>(pl.chunks[0] * 32);
-      ilu_.own_b = arena_.alloc<Vec4<double>>(pl.chunks[1] * 32);
-      h2d(ilu_.cl_pos, pl.pos[0], s);
-      for (auto* f : {k_ilu_sweep_cluster<true>, k_ilu_sweep_cluster<false>})
-        O2F_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem));
-    }
     ilu_.lo_cells = arena_.alloc<int32_t>(nc);
     ilu_.tmp = arena_.alloc<Vec4<double>>(nc);
     ilu_.sync = arena_.alloc<SweepSync>(2);
@@ -729,6 +709,7 @@ void Solver::ilu_factor() {
     sync();
     ilu_alloc_ = true;
   }
+  plan_sweeps();
   O2F_CUDA(cudaMemsetAsync(ilu_status_, 0, sizeof(int), s));
   if (full_jac())  // ILU(0) of the full operator on the first-order pattern
     k_ilu_assemble_full<<<grid(nc), kBlock, 0, s>>>(nc, fjac_off_, fjac_idx_, fjac_blk_, params_.adjoint_shift, ilu_);
@@ -766,8 +747,39 @@ void Solver::ilu_factor() {
 // out on none of the O-grids up to 2.0M cells).  Measured per adjoint
 // iteration alone, block / waiting: 0.35 / 1.4 ms at 5k rows, 1.1 / 5.2 at
 // 75k, 2.3 / 11.6 at 300k, 4.5 / 20.8 at 814k.
-bool Solver::ilu_block_sweeps() const {
-  return !ilu_waiting_ && ilu_plan_h_.cluster > 0 && params_.adjoint_sweeps != O2F_SWEEPS_WAITING;
+bool Solver::ilu_block_sweeps() const { return block_sweeps_wanted() && ilu_.cl_blocks > 0; }
+bool Solver::block_sweeps_wanted() const { return !ilu_waiting_ && params_.adjoint_sweeps != O2F_SWEEPS_WAITING; }
+
+// The block sweeps' plan, made at the first factorization that is for them: a
+// context that only steps in time, or that sweeps the other way, has no use
+// for it (21 ms at 74,528 rows, 108 at 300,300, and 1.2 KB a row on the
+// device).
+void Solver::plan_sweeps() {
+  if (ilu_planned_ || !block_sweeps_wanted()) return;
+  const int64_t nc = topo_.nc;
+  cudaStream_t s = stream_;
+  const SweepPlan pl = make_sweep_plan(nc, ilu_nbr_h_, ilu_pos_h_, ilu_order_h_);
+  if (pl.cluster > 0) {
+    for (int d = 0; d < 2; ++d) {
+      ilu_.cl_nlev[d] = pl.nlev[d];
+      ilu_.cl_chunks[d] = (int)pl.chunks[d];
+      ilu_.cl_info[d] = arena_.alloc<int32_t>(pl.info[d].size());
+      ilu_.cl_rec[d] = arena_.alloc<int32_t>(pl.rec[d].size());
+      ilu_.pack[d] = arena_.alloc<double>(pl.chunks[d] * 2048);
+      h2d(ilu_.cl_info[d], pl.info[d], s);
+      h2d(ilu_.cl_rec[d], pl.rec[d], s);
+    }
+    ilu_.cl_pos = arena_.alloc<int32_t>(nc);
+    ilu_.packD = arena_.alloc<double>(pl.chunks[1] * 512);
+    ilu_.own_f = arena_.alloc<Vec4<double>>(pl.chunks[0] * 32);
+    ilu_.own_b = arena_.alloc<Vec4<double>>(pl.chunks[1] * 32);
+    h2d(ilu_.cl_pos, pl.pos[0], s);
+    for (auto* f : {k_ilu_sweep_cluster<true>, k_ilu_sweep_cluster<false>})
+      O2F_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem));
+    sync();  // the plan's host arrays go out of scope
+    ilu_.cl_blocks = pl.cluster;
+  }
+  ilu_planned_ = true;
 }
 
 // z = M^{-1} r = U^{-1} L^{-1} r, one launch per triangle: a cluster of blocks

@@ -13,7 +13,6 @@
 #include "device_types.hpp"
 #include "mesh_host.hpp"
 #include "o2f.h"
-#include "sweep_plan.hpp"
 
 namespace o2f {
 
@@ -213,6 +212,8 @@ class Solver {
   void ilu_factor();
   void ilu_apply(const Vec4<double>* r, Vec4<double>* z, const int* gate);
   void ilu_check_sweeps();
+  void plan_sweeps();
+  bool block_sweeps_wanted() const;
   bool ilu_block_sweeps() const;  // the block sweeps, not the waiting ones
 
  public:
@@ -221,7 +222,7 @@ class Solver {
  private:
   std::vector<int32_t> ilu_nbr_h_, ilu_pos_h_, ilu_order_h_, lo_off_h_, lo_cells_h_, ilu_sweep_h_;
   int ilu_n_up_ = 0;  // levels of the backward sweep's dependencies
-  SweepPlan ilu_plan_h_;  // rows, levels and value routes of the block sweeps
+  bool ilu_planned_ = false;  // the block sweeps' plan has been made (ilu_.cl_blocks 0: there is none)
   bool ilu_waiting_ = false;  // test hook: use the sweeps that wait on other rows
   IluDev ilu_{};
   bool ilu_alloc_ = false;
