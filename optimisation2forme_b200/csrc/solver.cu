@@ -62,14 +62,24 @@ void validate_params(const o2f_params& p) {
   if (!(p.adjoint_shift >= 0.0) || !(p.adjoint_shift < 1e6)) throw Error(O2F_ERR_ARG, "adjoint_shift out of range");
 }
 
-// Cells per tile of the time loop's kernels (= threads per block), 0: the
-// separate kernels.  Up to here a step is bound by the latency of its
-// kernels, beyond it by their throughput, where the separate kernels run
-// with more warps.  Measured, us per FP64 step, tiles of 128 / separate:
-// 62 / 80 at 3,840 triangles, 80 / 105 at 74,528, 159 / 193 at 150,544,
-// 230 / 233 at 213,440, 344 / 320 at 300,300; tiles of 64 and 96 cells are
-// behind 128 at every size.  (FP32: 46 / 68, 60 / 84, 113 / 113, 154 / 133.)
-int tile_cells(int64_t nc) { return nc < 180000 ? kTileMax : 0; }
+// Whether the time loop of a mesh runs on tiles (of kTileMax cells, a thread
+// each) or on the separate kernels.  Up to here a step is bound by the latency
+// of its kernels, beyond it by their throughput, where the separate kernels
+// run with more warps.  Measured, us per step, tiles of 128 / separate: FP64
+// 62 / 80 at 3,840 triangles, 80 / 105 at 74,528, 136 / 160 at 123,120, 147 /
+// 186 at 151,360, 206 / 210 at 178,360, 230 / 233 at 213,440, 344 / 320 at
+// 300,300; tiles of 64 and 96 cells are behind 128 at every size.
+// FP32, whose separate kernels gain more from their warps: tiles are ahead
+// while the blocks the chip holds at once (four an SM) take them in one wave
+// (46 / 68 at 3,840, 60 / 84 at 74,528) or in two of which the second is
+// nearly full (99 / 103 at 140,280, 101 / 109 at 151,360), and behind with a
+// second wave less full (87 / 80 at 79,520, 93 / 85 at 103,360, 97 / 92 at
+// 123,120) or a third (136 / 116 at 167,088, 142 / 119 at 178,360).
+bool on_tiles(int64_t nc, bool fp32) {
+  if (!fp32) return nc < 180000;
+  const int64_t wave = 4 * 148 * kTileMax;
+  return nc <= wave || (4 * nc > 7 * wave && nc <= 2 * wave);
+}
 
 }  // namespace
 
@@ -347,7 +357,7 @@ void Solver::upload_mesh() {
   O2F_CUDA(cudaMemsetAsync(ks_, 0, sizeof(KrylovState), s));
   sync();  // host staging vectors go out of scope
   setup_ilu_host(jslot, ec, ebc);
-  if (tile_cells(nc) > 0) {  // for build_tiles
+  if (on_tiles(nc, false) || on_tiles(nc, true)) {  // for build_tiles
     slot_h_ = std::move(slot);
     ev_h_ = std::move(ev);
   }
@@ -1089,11 +1099,12 @@ void Solver::debug_get(const std::string& which, double* out) {
 
 // Tiles of consecutive cells with their vertices and edges, for meshes whose
 // time loop runs on them.
-void Solver::build_tiles() {
+void Solver::build_tiles(bool fp32) {
   const int64_t nc = topo_.nc;
   if (!norm_part_) norm_part_ = arena_.alloc<double>(grid(nc) * (kBlock / kTileMax));
-  const int T = tile_cells(nc);
-  if (tiles_ || T == 0) return;
+  tiled_ = on_tiles(nc, fp32);
+  if (tiles_ || !tiled_) return;
+  const int T = kTileMax;
   const int nt = (int)((nc + T - 1) / T);
   TileDev td{};
   td.n = nt;
@@ -1173,7 +1184,7 @@ void Solver::step_control(int stage) {
 
 void Solver::launch_stage(int stage, const RkStage& rk) {
   cudaStream_t s = stream_;
-  if (!tiles_) {
+  if (!tiled_) {
     const Topo& t = topo_;
     const Geom<double>& g = geom_;
     const Work<double>& w = work_;
@@ -1237,7 +1248,7 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
   st.drop_tol = drop_tol;
   st.max_steps = max_steps;
   O2F_CUDA(cudaMemcpyAsync(step_, &st, sizeof(st), cudaMemcpyHostToDevice, stream_));
-  build_tiles();
+  build_tiles(f32());
   const double* dt = &step_->dt;
   const RkStage s1{0.0, 1.0, dt, 1, norm_part_};
   const RkStage s2{3.0 / 4.0, 1.0 / 4.0, dt, 0, nullptr};
@@ -1281,7 +1292,7 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
     while (true) {
       O2F_CUDA(cudaGraphLaunch(exec, stream_));
       launched += kStepsPerGraph;
-      launches_ += kStepsPerGraph * (tiles_ ? 6 : 17);
+      launches_ += kStepsPerGraph * (tiled_ ? 6 : 17);
       if (launched % (kStepsPerGraph * 4) == 0 || launched >= max_steps) {
         O2F_CUDA(cudaMemcpyAsync(host_st, step_, sizeof(StepState), cudaMemcpyDeviceToHost, stream_));
         sync();
@@ -1308,7 +1319,7 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
     launch_residual(geom_, work_, Ukeep_, nullptr, false, nullptr);
     sync();
   }
-  if (!mixed && tiles_ && (fin.step > 0 || fin.stop == 2)) publish_stage(fin.stop == 2);
+  if (!mixed && tiled_ && (fin.step > 0 || fin.stop == 2)) publish_stage(fin.stop == 2);
   have_residual_ = fin.step > 0;
   invalidate_linearisation();
   if (fin.stop == 2) throw Error(O2F_ERR_NONFINITE, "non-finite state or residual in the time loop");

@@ -130,7 +130,7 @@ class Solver {
   void launch_stage(int stage, const RkStage& rk);
   void launch_stage_f32(int stage, const RkStage& rk);
   void step_control(int stage);
-  void build_tiles();
+  void build_tiles(bool fp32);
   void tile_smem_f32();
   void publish_stage(bool first_stage);
   void build_jt_blocks();
@@ -190,6 +190,7 @@ class Solver {
   float* blk32_ = nullptr;
   double* norm_part_ = nullptr;
   std::unique_ptr<TileDev> tiles_;  // tiles of the time loop's kernels
+  bool tiled_ = false;              // the present time loop runs on them
   std::vector<int32_t> slot_h_;     // host copies for them, until they are built
   std::vector<int2> ev_h_;
   StepState* step_ = nullptr;

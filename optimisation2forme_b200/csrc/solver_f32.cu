@@ -240,7 +240,7 @@ void Solver::launch_stage_f32(int stage, const RkStage& rk) {
   const Work<float>& w = work32_;
   cudaStream_t s = stream_;
   StepState* st = step_;
-  if (tiles_) {
+  if (tiled_) {
     const TileDev& td = *tiles_;
     O2F_CUDA(tile_launch(k_tile_gradient<float>, td, tile_gradient_smem<float>(td), s, td, t, g, U32_, phys_, w, nullptr,
                          &st->stop));
