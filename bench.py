@@ -597,7 +597,7 @@ def run_candidates(args, rank: int, world: int) -> dict | None:
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         try:
             line["cpu_baseline"] = cpu_baseline(args, cands[0], rk, plain_out[0]["iters"])
-        except FileNotFoundError as err:  # the line stands without it
+        except ReferenceMissing as err:  # the line stands without it
             line["cpu_baseline"] = {"unavailable": str(err)}
     return line if rank == 0 else None
 
@@ -664,6 +664,10 @@ def run_large(args, rank: int, world: int) -> dict | None:
 # ---------------------------------------------------------------------------
 # The reference's CPU code (oracle/_ref)
 
+class ReferenceMissing(RuntimeError):
+    """The reference's own code has not been built here."""
+
+
 def reference_eval(c: Candidate, steps: int, iters: int, threads: int) -> dict:
     """One reduced evaluation of the reference's own code on candidate c:
     `steps` SSP-RK3 steps, J and the adjoint right-hand side, `iters`
@@ -671,7 +675,7 @@ def reference_eval(c: Candidate, steps: int, iters: int, threads: int) -> dict:
     timed by phase inside the process (the mesh build is not timed)."""
     from oracle import ref
     if not ref.EXE_FAST.exists():
-        raise FileNotFoundError("reference build oracle/_ref is not present")
+        raise ReferenceMissing("reference build oracle/_ref is not present")
     with tempfile.TemporaryDirectory() as td:
         td = Path(td)
         ref.write_binary_mesh(td / "mesh.bin", c.mesh)
@@ -793,7 +797,7 @@ def main() -> int:
         if args.impl == "reference":
             try:
                 line = run_reference(args, rank, world)
-            except FileNotFoundError as err:
+            except ReferenceMissing as err:
                 line = {"impl": "reference", "unavailable": str(err)}
         elif args.workload == "large":
             line = run_large(args, rank, world)
