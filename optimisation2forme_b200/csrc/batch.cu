@@ -183,9 +183,9 @@ void Batch::tune(int reps, int* cfg_out) {
     if (f32_) {
       s->ensure_f32();
       s->f32_state_sync();
-      s->launch_residual_f32(nullptr, nullptr);
+      s->launch_residual_f32();
     } else {
-      s->launch_residual(s->geom_, s->work_, s->U_, nullptr, false, nullptr);
+      s->launch_residual(s->geom_, s->work_, s->U_, false);
     }
   }
   static const int kBlocks[] = {128, 256, 512};
@@ -297,7 +297,7 @@ void Batch::rk3_run(int64_t max_steps, double drop_tol, int64_t* steps_done, dou
     if (status) status[i] = host[i].stop == 2 ? O2F_ERR_NONFINITE : O2F_OK;
     // FP32 contexts: the linearisation's FP64 interface states about the
     // last stage's input state, as Solver::rk3_run leaves them.
-    if (f32_ && host[i].step > 0) s.launch_residual(s.geom_, s.work_, s.Ukeep_, nullptr, false, nullptr);
+    if (f32_ && host[i].step > 0) s.launch_residual(s.geom_, s.work_, s.Ukeep_, false);
     s.have_residual_ = host[i].step > 0;
     s.invalidate_linearisation();
   }

@@ -937,22 +937,14 @@ __device__ __forceinline__ double cell_residual_at(int64_t c, int64_t nc, const 
   return cell_residual_from<T, kRk>(c, nc, slot, g.cgeom, EdgeFluxes<T>{g.egeom, F, etq, etqy}, U, Uold, R, rk);
 }
 
-template <typename T, bool kRk>
+template <typename T>
 __global__ void __launch_bounds__(kBlock) k_cell_residual(int64_t nc, const int32_t* __restrict__ slot, Geom<T> g,
                                                           const Vec4<T>* __restrict__ F,
                                                           const Vec4<T>* __restrict__ etq,
                                                           const T* __restrict__ etqy, Vec4<T>* __restrict__ U,
-                                                          Vec4<T>* __restrict__ Uold, Vec4<T>* __restrict__ R,
-                                                          RkStage rk, const int* gate) {
-  __shared__ double smem[kBlock / 32];
-  if (gated(gate)) return;
+                                                          Vec4<T>* __restrict__ R) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double r2 = 0.0;
-  if (c < nc) r2 = cell_residual_at<T, kRk>(c, nc, slot, g, F, etq, etqy, U, Uold, R, rk);
-  if (kRk && rk.norm_part) {
-    const double s = block_sum(r2, smem);
-    if (threadIdx.x == 0) rk.norm_part[blockIdx.x] = s;
-  }
+  if (c < nc) cell_residual_at<T, false>(c, nc, slot, g, F, etq, etqy, U, nullptr, R, RkStage{});
 }
 
 }  // namespace o2f

@@ -128,21 +128,13 @@ __device__ __forceinline__ double cell_residual_mixed_at(
                                        rk, dtp, keep);
 }
 
-template <bool kRk>
 __global__ void __launch_bounds__(kBlock) k_cell_residual_mixed(
     int64_t nc, const int32_t* __restrict__ slot, Geom<float> g, const Vec4<float>* __restrict__ F,
     const Vec4<float>* __restrict__ etq, const float* __restrict__ etqy, Vec4<float>* __restrict__ U32,
-    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ Uold, Vec4<double>* __restrict__ R, RkStage rk,
-    Vec4<double>* __restrict__ keep, const int* gate) {
-  __shared__ double smem[kBlock / 32];
-  if (gated(gate)) return;
+    Vec4<double>* __restrict__ U, Vec4<double>* __restrict__ R) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double r2 = 0.0;
-  if (c < nc) r2 = cell_residual_mixed_at<kRk>(c, nc, slot, g, F, etq, etqy, U32, U, Uold, R, rk, rk.dt, keep);
-  if (kRk && rk.norm_part) {
-    const double s = block_sum(r2, smem);
-    if (threadIdx.x == 0) rk.norm_part[blockIdx.x] = s;
-  }
+  if (c < nc)
+    cell_residual_mixed_at<false>(c, nc, slot, g, F, etq, etqy, U32, U, nullptr, R, RkStage{}, nullptr, nullptr);
 }
 
 }  // namespace o2f

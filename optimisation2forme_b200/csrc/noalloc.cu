@@ -7,8 +7,8 @@
 // library a fixed device-memory budget, or owns all device memory through
 // its own pool, cannot let a call allocate at all.
 //
-// This is a variant of the time loop's norm reduction (k_cell_residual's
-// per-block partial sums of R_rho^2, folded by k_step_norm), whose partial
+// This is a variant of the time loop's norm reduction (the first stage's
+// per-block partial sums of R_rho^2, folded by step_norm_block), whose partial
 // sums live in context memory.  Here the reduction's scratch -- a completion
 // ticket, the result slot and the per-block partial sums -- is one file-scope
 // static device array of kNormScratchBytes (33,280 bytes), so the call needs
@@ -145,10 +145,10 @@ void Solver::residual_norm_noalloc(double* norm_out) {
                   "(it allocates the FP32 buffers)");
     ensure_f32();
     f32_state_sync();
-    launch_residual_f32(nullptr, nullptr);
+    launch_residual_f32();
     f32_publish_interfaces();
   } else {
-    launch_residual(geom_, work_, U_, nullptr, true, nullptr);
+    launch_residual(geom_, work_, U_, true);
   }
   have_residual_ = true;
   invalidate_linearisation();

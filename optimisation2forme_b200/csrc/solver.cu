@@ -498,7 +498,7 @@ void Solver::render_field(const std::string& field, int nx, int ny, const std::s
   // the gradient fields read the Green-Gauss gradients of a residual of the current state
   const bool needs_grad = f >= kFieldUx && f <= kFieldDiv;
   if (needs_grad) {
-    launch_residual(geom_, work_, U_, nullptr, true, nullptr);
+    launch_residual(geom_, work_, U_, true);
     have_residual_ = true;
   }
   if (!render_scalar_) {
@@ -922,8 +922,10 @@ void Solver::cell_permutation(int64_t* new_of_old) const {
   std::memcpy(new_of_old, cinv_.data(), cinv_.size() * sizeof(int64_t));
 }
 
-void Solver::launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, const int* gate,
-                             bool write_grad, const void* rkp, int alpha_mode) {
+// Everything of a residual but its last kernel: vertex states, gradients and
+// interface states, viscous terms, fluxes.
+void Solver::launch_fluxes(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, const int* gate,
+                           bool write_grad, int alpha_mode) {
   const Topo& t = topo_;
   cudaStream_t s = stream_;
   k_vertex_state<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U, phys_, w.vq, gate);
@@ -934,23 +936,21 @@ void Solver::launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<
     k_cell_gradient_alpha<2><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_, w.eL,
                                                             w.eR, w.ctq, w.ctqy, fjac_alpha_);
   else if (write_grad)
-    k_cell_gradient<double, true><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_,
-                                                                w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
+    k_cell_gradient<double, true><<<grad_grid(t.nc), kGradBlock, 0, s>>>(
+        t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_, w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
   else
-    k_cell_gradient<double, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_,
-                                                                 w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
+    k_cell_gradient<double, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(
+        t.nc, t.slot, g, t.ev, t.ec, t.ebc, U, w.vq, phys_, w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
   k_vertex_visc<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq,
                                                       w.vtqy, gate);
   k_edge_flux<double><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F,
                                                     w.etq, w.etqy, gate);
-  if (rkp) {
-    const RkStage rk = *static_cast<const RkStage*>(rkp);
-    k_cell_residual<double, true><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U, Uold_, w.R,
-                                                                rk, gate);
-  } else {
-    k_cell_residual<double, false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U, Uold_,
-                                                                 w.R, RkStage{}, gate);
-  }
+}
+
+void Solver::launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, bool write_grad,
+                             int alpha_mode) {
+  launch_fluxes(g, w, U, nullptr, write_grad, alpha_mode);
+  k_cell_residual<double><<<grid(topo_.nc), kBlock, 0, stream_>>>(topo_.nc, topo_.slot, g, w.F, w.etq, w.etqy, U, w.R);
   launches_ += 5;
   O2F_CUDA(cudaGetLastError());
 }
@@ -963,9 +963,9 @@ void Solver::residual(double* R_ref) {
   }
   O2F_CUDA(cudaEventRecord(ev0_, stream_));
   if (f32())
-    launch_residual_f32(nullptr, nullptr);
+    launch_residual_f32();
   else
-    launch_residual(geom_, work_, U_, nullptr, true, nullptr);
+    launch_residual(geom_, work_, U_, true);
   O2F_CUDA(cudaEventRecord(ev1_, stream_));
   if (f32()) f32_publish_interfaces();
   sync();
@@ -984,7 +984,7 @@ void Solver::profile_kernels(int reps, double* ms_out) {
   const Geom<double>& g = geom_;
   const Work<double>& w = work_;
   cudaStream_t s = stream_;
-  launch_residual(geom_, work_, U_, nullptr, false, nullptr);  // fresh interface states
+  launch_residual(geom_, work_, U_, false);  // fresh interface states
   have_residual_ = true;
   invalidate_linearisation();
   build_jt_blocks();
@@ -994,7 +994,7 @@ void Solver::profile_kernels(int reps, double* ms_out) {
   if (f32()) {  // the residual kernels of this context's precision
     ensure_f32();
     f32_state_sync();
-    launch_residual_f32(nullptr, nullptr);
+    launch_residual_f32();
   }
   for (int k = 0; k < O2F_K_COUNT; ++k) {
     O2F_CUDA(cudaEventRecord(ev0_, s));
@@ -1022,8 +1022,7 @@ void Solver::profile_kernels(int reps, double* ms_out) {
                                                             w.F, w.etq, w.etqy, nullptr);
           break;
         case O2F_K_CELL_RESIDUAL:
-          k_cell_residual<double, false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U_,
-                                                                       Uold_, w.R, RkStage{}, nullptr);
+          k_cell_residual<double><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U_, w.R);
           break;
         case O2F_K_JT_APPLY:
           jt_apply_dev(s_, tmp_);
@@ -1186,18 +1185,9 @@ void Solver::launch_stage(int stage, const RkStage& rk) {
   cudaStream_t s = stream_;
   if (!tiled_) {
     const Topo& t = topo_;
-    const Geom<double>& g = geom_;
-    const Work<double>& w = work_;
-    const int* gate = &step_->stop;
-    k_vertex_state<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U_, phys_, w.vq, gate);
-    k_cell_gradient<double, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(
-        t.nc, t.slot, g, t.ev, t.ec, t.ebc, U_, w.vq, phys_, w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
-    k_vertex_visc<double><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
-                                                        gate);
-    k_edge_flux<double><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F,
-                                                      w.etq, w.etqy, gate);
+    launch_fluxes(geom_, work_, U_, &step_->stop, false, 0);
     auto* last = stage == 1 ? k_cell_residual_stage<1> : stage == 2 ? k_cell_residual_stage<2> : k_cell_residual_stage<3>;
-    last<<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, phys_, w, U_, Uold_, rk, norm_part_, step_);
+    last<<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, geom_, phys_, work_, U_, Uold_, rk, norm_part_, step_);
     step_control(stage);
     O2F_CUDA(cudaGetLastError());
     return;
@@ -1316,7 +1306,7 @@ void Solver::rk3_run(int64_t max_steps, double drop_tol, double* history, int64_
   // right-hand side linearise about the last stage's input state, as in the
   // FP64 path; one FP64 residual of that state gives its interface states.
   if (mixed && fin.step > 0) {
-    launch_residual(geom_, work_, Ukeep_, nullptr, false, nullptr);
+    launch_residual(geom_, work_, Ukeep_, false);
     sync();
   }
   if (!mixed && tiled_ && (fin.step > 0 || fin.stop == 2)) publish_stage(fin.stop == 2);
@@ -1441,19 +1431,19 @@ void Solver::build_full_jacobian() {
   // frozen limiter: the limiter values of the current state, held in every
   // perturbed residual
   const int amode = params_.adjoint_jacobian == O2F_JAC_FROZEN ? 2 : 0;
-  if (amode) launch_residual(geom_, work_, U_, nullptr, false, nullptr, 1);
+  if (amode) launch_residual(geom_, work_, U_, false, 1);
   const int64_t ncol = (int64_t)fjac_coff_h_.size() - 1;
   for (int64_t col = 0; col < ncol; ++col) {
     const int32_t* cells = fjac_ccells_ + fjac_coff_h_[col];
     const int64_t n = fjac_coff_h_[col + 1] - fjac_coff_h_[col];
     for (int k = 0; k < 4; ++k) {
       k_fjac_perturb<<<grid(n), kBlock, 0, st>>>(n, cells, U_, fjac_Up_, k, 1.0, e);
-      launch_residual(geom_, work_, fjac_Up_, nullptr, false, nullptr, amode);
+      launch_residual(geom_, work_, fjac_Up_, false, amode);
       O2F_CUDA(cudaMemcpyAsync(fjac_Rp_, work_.R, nc * sizeof(Vec4<double>), cudaMemcpyDeviceToDevice, st));
       if (nw) k_fjac_wall_terms<<<grid(nw), kBlock, 0, st>>>(nw, topo_.wall_edges, geom_, work_.eL, work_.etq, ph,
                                                               fjac_tlp_, fjac_tdp_);
       k_fjac_perturb<<<grid(n), kBlock, 0, st>>>(n, cells, U_, fjac_Up_, k, -1.0, e);
-      launch_residual(geom_, work_, fjac_Up_, nullptr, false, nullptr, amode);
+      launch_residual(geom_, work_, fjac_Up_, false, amode);
       if (nw) k_fjac_wall_terms<<<grid(nw), kBlock, 0, st>>>(nw, topo_.wall_edges, geom_, work_.eL, work_.etq, ph,
                                                               fjac_tlm_, fjac_tdm_);
       k_fjac_extract<<<grid(n), kBlock, 0, st>>>(n, cells, fjac_off_, fjac_idx_, U_, fjac_Rp_, work_.R, k, e,
@@ -1467,7 +1457,7 @@ void Solver::build_full_jacobian() {
     }
   }
   // the residual and interface states of the state itself
-  launch_residual(geom_, work_, U_, nullptr, false, nullptr);
+  launch_residual(geom_, work_, U_, false);
   O2F_CUDA(cudaGetLastError());
   sync();
   have_residual_ = true;
@@ -1751,14 +1741,14 @@ void Solver::shape_gradient(const o2f_shape_params& sp, const int* ids, int n, d
     throw Error(O2F_ERR_STATE, "no adjoint solution: solve first or pass lambda");
   }
   // computeShapeGradient starts with a residual of the unperturbed mesh (:955-956).
-  launch_residual(geom_, work_, U_, nullptr, false, nullptr);
+  launch_residual(geom_, work_, U_, false);
   have_residual_ = true;
   invalidate_linearisation();
   for (int k = 0; k < n; ++k) {
     double J[2];
     for (int sgn = 0; sgn < 2; ++sgn) {
       perturbed_geometry(sp, ids[k], sgn == 0 ? eps : -eps);
-      launch_residual(pgeom_, pwork_, U_, nullptr, false, nullptr);
+      launch_residual(pgeom_, pwork_, U_, false);
       k_forces<double><<<1, kBlock, 0, stream_>>>(topo_.n_wall, topo_.wall_edges, pgeom_, pwork_.eL, pwork_.etq,
                                                   phys_, beta, scal_ + 4 + 4 * sgn);
       if (sgn == 0)

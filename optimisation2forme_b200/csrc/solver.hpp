@@ -124,8 +124,10 @@ class Solver {
   void compute_phys();
   // alpha_mode 1 / 2: record / hold the limiter values in fjac_alpha_
   // (the frozen-limiter linearisation); 0 everywhere else.
-  void launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, const int* gate,
-                       bool write_grad, const void* rk, int alpha_mode = 0);
+  void launch_residual(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, bool write_grad,
+                       int alpha_mode = 0);
+  void launch_fluxes(const Geom<double>& g, const Work<double>& w, Vec4<double>* U, const int* gate, bool write_grad,
+                     int alpha_mode);
   // One RK3 stage of the time loop (kernels_tile.cuh).
   void launch_stage(int stage, const RkStage& rk);
   void launch_stage_f32(int stage, const RkStage& rk);
@@ -156,7 +158,8 @@ class Solver {
   void ensure_f32();
   void f32_state_sync();
   void f32_publish_interfaces();
-  void launch_residual_f32(const int* gate, const void* rk, Vec4<double>* keep = nullptr);
+  void launch_residual_f32();
+  void launch_fluxes_f32(const int* gate);
   void profile_kernel_f32(int k);  // one launch of residual kernel class k (O2F_K_*) in FP32
   void f32_blocks();
   void to_internal(const double* ref, Vec4<double>* dev);

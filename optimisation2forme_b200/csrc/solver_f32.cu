@@ -203,26 +203,25 @@ void Solver::f32_publish_interfaces() {
   O2F_CUDA(cudaGetLastError());
 }
 
-void Solver::launch_residual_f32(const int* gate, const void* rkp, Vec4<double>* keep) {
+void Solver::launch_fluxes_f32(const int* gate) {
   const Topo& t = topo_;
   const Geom<float>& g = geom32_;
   const Work<float>& w = work32_;
   cudaStream_t s = stream_;
   k_vertex_state<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U32_, phys_, w.vq, gate);
-  k_cell_gradient<float, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
-                                                              w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
+  k_cell_gradient<float, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(
+      t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_, w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
   k_vertex_visc<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
                                                      gate);
   k_edge_flux<float><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F, w.etq,
                                                    w.etqy, gate);
-  if (rkp) {
-    const RkStage rk = *static_cast<const RkStage*>(rkp);
-    k_cell_residual_mixed<true><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U32_, U_, Uold_,
-                                                              work_.R, rk, keep, gate);
-  } else {
-    k_cell_residual_mixed<false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U32_, U_, Uold_,
-                                                               work_.R, RkStage{}, nullptr, gate);
-  }
+}
+
+void Solver::launch_residual_f32() {
+  const Work<float>& w = work32_;
+  launch_fluxes_f32(nullptr);
+  k_cell_residual_mixed<<<grid(topo_.nc), kBlock, 0, stream_>>>(topo_.nc, topo_.slot, geom32_, w.F, w.etq, w.etqy, U32_,
+                                                                U_, work_.R);
   launches_ += 5;
   O2F_CUDA(cudaGetLastError());
 }
@@ -251,14 +250,7 @@ void Solver::launch_stage_f32(int stage, const RkStage& rk) {
                          stage == 3 ? Ukeep_ : nullptr, norm_part_, hist_dev_, st));
     return;
   }
-  const int* gate = &st->stop;
-  k_vertex_state<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, U32_, phys_, w.vq, gate);
-  k_cell_gradient<float, false><<<grad_grid(t.nc), kGradBlock, 0, s>>>(t.nc, t.slot, g, t.ev, t.ec, t.ebc, U32_, w.vq, phys_,
-                                                             w.eL, w.eR, w.ctq, w.ctqy, w.grad, gate);
-  k_vertex_visc<float><<<grid(t.nv), kBlock, 0, s>>>(t.nv, t.voff, t.vcid, g.vw, t.vbc, w.ctq, w.ctqy, w.vtq, w.vtqy,
-                                                     gate);
-  k_edge_flux<float><<<grid(t.ne), kBlock, 0, s>>>(t.ne, g, t.ev, t.ebc, w.eL, w.eR, w.vtq, w.vtqy, phys_, w.F, w.etq,
-                                                   w.etqy, gate);
+  launch_fluxes_f32(&st->stop);
   auto* last = stage == 1   ? k_cell_residual_mixed_stage<1>
                : stage == 2 ? k_cell_residual_mixed_stage<2>
                             : k_cell_residual_mixed_stage<3>;
@@ -290,8 +282,7 @@ void Solver::profile_kernel_f32(int k) {
                                                        w.etq, w.etqy, nullptr);
       break;
     case O2F_K_CELL_RESIDUAL:
-      k_cell_residual_mixed<false><<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U32_, U_, Uold_,
-                                                                 work_.R, RkStage{}, nullptr, nullptr);
+      k_cell_residual_mixed<<<grid(t.nc), kBlock, 0, s>>>(t.nc, t.slot, g, w.F, w.etq, w.etqy, U32_, U_, work_.R);
       break;
     default:
       break;
