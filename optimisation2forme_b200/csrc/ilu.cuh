@@ -472,13 +472,6 @@ static_assert(kSweepSmem <= 227 * 1024, "block sweep shared memory above the per
 static_assert(kStageBwdD + kStageChunksBwd * 512 <= kStageDoubles, "backward staging overflows its buffer");
 constexpr int kSweepWaitLimit = 1 << 20;  // polls of an mbarrier (up to 1 us each) before the sweep gives up
 
-// Place of element el of the block at lane q inside its 512 doubles: the two
-// halves of a block row, then (row, component), so that a warp's four lanes
-// per row read 16 consecutive bytes each, all 32 lanes 512.
-__host__ __device__ __forceinline__ int sweep_pack_place(int q, int el) {
-  return ((el >> 1) & 1) * 256 + (q * 4 + (el >> 2)) * 2 + (el & 1);
-}
-
 // Factor blocks in sweep order, repacked after every factorization: dependency
 // d of position p of direction dir at pack[dir] + (p >> 5) * 2048 + d * 512 +
 // sweep_pack_place(p & 31, .), D^-1 of backward position p at packD +

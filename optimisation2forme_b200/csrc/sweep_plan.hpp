@@ -37,6 +37,12 @@
 #include <cstdint>
 #include <vector>
 
+#if defined(__CUDACC__)
+#define O2F_PLAN_FN __host__ __device__ __forceinline__
+#else
+#define O2F_PLAN_FN inline
+#endif
+
 namespace o2f {
 
 constexpr int kSweepChunks = 2;                // 32-row chunks of a level per thread block
@@ -58,6 +64,14 @@ struct SweepPlan {
   std::vector<int32_t> rec[2];        // [32 * chunks * kSweepRec]
   std::vector<int32_t> pos[2];        // [n] position of each row
 };
+
+// Place of element el of the 4x4 block of row q of a chunk inside the 512
+// doubles of the chunk's blocks: the two halves of a block row, then (row,
+// component), so that a warp's four lanes
+// per row read 16 consecutive bytes each, all 32 lanes 512.
+O2F_PLAN_FN int sweep_pack_place(int q, int el) {
+  return ((el >> 1) & 1) * 256 + (q * 4 + (el >> 2)) * 2 + (el & 1);
+}
 
 // Thread blocks per cluster: enough for the mean level in one round with a
 // quarter to spare, so that the cap costs no levels.
