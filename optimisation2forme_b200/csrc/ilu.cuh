@@ -554,6 +554,7 @@ struct SweepWaits {
       if (bar_try(bar, parity)) return;
     bad = true;
     *quit = 1;
+    __threadfence_block();  // before the next cluster barrier
   }
 };
 
@@ -657,8 +658,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       // A level's barrier is set kSweepNear levels ahead: by then every warp
       // has left the level that used it last (kSweepSkew levels back), so a
       // phase that has nothing to wait for cannot pass one that is waited on.
-      // (That level's phase is over then, unless a value was held back: it is
-      // looked at, since a phase must not be set twice.)
+      // (And that level's phase is over then, unless a warp gave up on it: it
+      // marked that before it came to the cluster barrier.  A phase must not be
+      // set twice.)
       const bool arms = slot == kStageRing;
       const int kLead = arms ? kSweepNear : kL2Lead;
       auto work = [&](int l, const int4& in) {
@@ -684,9 +686,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_ilu_sweep_cluster(IluDev i
       for (int l = 0; l < nlev; ++l) {
         keep_together(l);
         const int4 in = entry(l + kLead);
-        const int last = arms ? l + kSweepNear - kSweepBars : l;
-        if (last >= 0) wait(bar_op + 8u * (last % kSweepBars), (last / kSweepBars) & 1);
-        wait.bad = __any_sync(0xffffffffu, bad);
+        if (arms) {
+          if (l % (kSweepSkew / 2) == 0 && *wait.quit) wait.bad = true;
+        } else {
+          wait(bar_op + 8u * (l % kSweepBars), (l / kSweepBars) & 1);
+          wait.bad = __any_sync(0xffffffffu, bad);
+        }
         if (!bad) work(l + kLead, in);
       }
     }

@@ -67,8 +67,8 @@ struct SweepPlan {
 
 // Place of element el of the 4x4 block of row q of a chunk inside the 512
 // doubles of the chunk's blocks: the two halves of a block row, then (row,
-// component), so that a warp's four lanes
-// per row read 16 consecutive bytes each, all 32 lanes 512.
+// component), so that a warp's four lanes per row read 16 consecutive bytes
+// each, all 32 lanes 512.
 O2F_PLAN_FN int sweep_pack_place(int q, int el) {
   return ((el >> 1) & 1) * 256 + (q * 4 + (el >> 2)) * 2 + (el & 1);
 }

@@ -145,6 +145,9 @@ static int simulate(const SweepPlan& pl, int dir, std::mt19937& rng, int held, i
       if (a.level % (kSweepSkew / 2) == 0) {
         if (a.level > 0 && !all_arrived(a.level / (kSweepSkew / 2))) continue;
         ++a.arrivals;
+#ifndef ARM_UNSEEN
+        if (w == kSolve + kRing && B.quit) a.bad = true;
+#endif
       }
       a.step = 1;
     } else if (l >= nlev) {
@@ -166,10 +169,6 @@ static int simulate(const SweepPlan& pl, int dir, std::mt19937& rng, int held, i
         if (!wait(a, B, B.empty[l % kRing], l / kRing)) continue;
         if (!a.bad) stage(B, l + kRing);
       } else {
-#ifndef ARM_UNSEEN
-        const int last = l + kSweepNear - kSweepBars;
-        if (last >= 0 && !wait(a, B, B.op[last % kSweepBars], last / kSweepBars)) continue;
-#endif
         if (!a.bad) arm(b, l + kSweepNear);
       }
       a.step = 2;
