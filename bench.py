@@ -69,9 +69,9 @@ NAMES = ["m", "p", "t"]
 
 # DRAM bytes per launch of k_cell_gradient (FP64) per cell: dram__bytes_read
 # + dram__bytes_write of one ncu capture on the 1,014,040-cell mesh
-# (`--workload kernels --mesh medium`, 329,626,368 B), scaled by cells to the
+# (`--workload kernels --mesh medium`, 318,958,336 B), scaled by cells to the
 # 2.0M mesh.
-TRAFFIC_PER_CELL = {"cell_gradient": 329_626_368 / 1_014_040}
+TRAFFIC_PER_CELL = {"cell_gradient": 318_958_336 / 1_014_040}
 
 
 def naca_name(spec) -> str:

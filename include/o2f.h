@@ -415,7 +415,10 @@ int o2f_mlp_n_params(o2f_mlp* net, int64_t* n);
 /* Copies a training set to the device: inputs [n*7], targets [n*8]. */
 int o2f_mlp_set_data(o2f_mlp* net, const float* inputs, const float* targets, int64_t n);
 /* `steps` Adam steps on seeded minibatches of `batch` points; loss_history
- * (may be NULL) receives the minibatch MSE of each step. */
+ * (may be NULL) receives the minibatch MSE of each step.  The gradients' sums
+ * over a batch have a fixed order up to 4,096 points, so equal calls on equal
+ * states give equal weights, bit for bit (larger batches add parts of the
+ * weight gradients in the order they come in; the loss history always does). */
 int o2f_mlp_train(o2f_mlp* net, int steps, int batch, float lr, uint64_t seed, float* loss_history);
 int o2f_mlp_predict(o2f_mlp* net, const float* inputs, int64_t n, float* outputs);
 /* Gradient of the MSE on one batch (n <= max_batch) without an update:

@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kSweepBlock) k_ilu_sweep(int n, IluDev ilu, co
 // Four lanes solve a row (one component each), eight warps the kSweepChunks
 // chunks of a block.  The arithmetic of a row (dependencies in slot order)
 // is that of k_ilu_sweep: both give the same bits.
-// Measured on B200, ms per adjoint iteration (four sweeps) alone: 0.96 at
+// Measured on B200, ms per adjoint iteration (four sweeps) alone: 0.97 at
 // 74,528 rows, 1.96 at 300,300, against 3.93 and 13.1 for one block walking
 // plain levels behind a block barrier and 5.2 and 11.6 for k_ilu_sweep, 1.09
 // and 2.31 with one set of warps and one staging warp per chunk.  About 900

@@ -755,8 +755,8 @@ void Solver::ilu_factor() {
 
 // O2F_SWEEPS_AUTO: block sweeps wherever they have a plan (operand slots ran
 // out on none of the O-grids up to 2.0M cells).  Measured per adjoint
-// iteration alone, block / waiting: 0.35 / 1.4 ms at 5k rows, 1.1 / 5.2 at
-// 75k, 2.3 / 11.6 at 300k, 4.5 / 20.8 at 814k.
+// iteration alone, block / waiting: 0.31 / 1.35 ms at 5k rows, 0.97 / 5.3 at
+// 75k, 1.96 / 11.5 at 300k, 3.85 / 20.8 at 814k.
 bool Solver::ilu_block_sweeps() const { return block_sweeps_wanted() && ilu_.cl_blocks > 0; }
 bool Solver::block_sweeps_wanted() const { return !ilu_waiting_ && params_.adjoint_sweeps != O2F_SWEEPS_WAITING; }
 
