@@ -7,7 +7,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
-from test_gpu_mlp import _inputs, _layer_slices
+from test_gpu_mlp import TOL_GRAD, _inputs, _layer_slices
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +41,20 @@ def test_training_gives_the_same_weights_every_time():
             runs.append(net.params()[0])
     assert np.array_equal(runs[0].view(np.int32), runs[1].view(np.int32))
     assert np.array_equal(runs[0].view(np.int32), runs[2].view(np.int32))
+
+
+# parts of one, two and three accumulators, with ragged last chunks
+@pytest.mark.parametrize("n", [577, 2047, 2049, 2177, 4096, 4111])
+def test_gradients_of_large_batches_match_the_oracle(n):
+    from optimisation2forme_b200.warmstart import Network
+    from oracle import mlp_ref
+    x = _inputs(n, n)
+    t = np.random.default_rng(n).standard_normal((n, 8)).astype(np.float32)
+    with Network(max_batch=4224, seed=9) as net:
+        loss, g = net.gradients(x, t)
+        p, f = net.params()
+    lo, go = mlp_ref.gradients(p, f, x, t)
+    assert abs(loss - lo) <= 1e-3 * lo
+    for s in _layer_slices():
+        den = np.linalg.norm(go[s])
+        assert np.linalg.norm(g[s] - go[s]) <= TOL_GRAD * den + (den == 0.0) * 1e-12
